@@ -1,24 +1,40 @@
 // e2d_mlp_deep.cu — the deep warm-start network on the tensor cores: 5 input
 // features (padded to 16), four hidden layers of 256 units with GELU (tanh
-// form), 4 outputs (padded to 16).  The network runs layer by layer over a
-// batch of rows, a layer's activations in HBM between kernels:
+// form), 4 outputs (padded to 16).
 //
-//   dense_kernel<FWD_GELU>   Z = A W^T + b (FP32, kept for the backward pass),
-//                            H = bf16(gelu(Z))
-//   dense_kernel<FWD_LINEAR> Y = A W^T + b                       (output layer)
-//   dense_kernel<BWD_GELU>   dZp = bf16((dZ W) * gelu'(Zp))      (W^T staged)
-//   dw_kernel                dW = dZ^T A over a CTA's rows -> its slot; the
-//                            slots are summed in CTA order (deterministic)
+//   net_kernel<false>  rows -> outputs: all five layers of a 128-row tile in one
+//                      kernel, the activations in shared memory between layers
+//   net_kernel<true>   forward, loss and the deltas of every layer of a tile,
+//                      leaving activations and deltas (BF16) for dw_kernel
+//   dw_kernel          every layer's weight and bias gradients from them
+//   adam_kernel        the update, and the BF16 copies of the new weights
+//
+// A pair of CTAs (a cluster) shares a tile: each computes 128 of a layer's
+// 256 columns, so its half of the weights (64 KB) and two activation buffers
+// (64 KB each) fit one SM, and writes its half of the next activations into
+// both CTAs' shared memory.  The 64 tiles of an 8,192-row minibatch thus use
+// 128 SMs.  What bounds net_kernel is the epilogue: tanhf and the GELU
+// arithmetic, about 34 instructions per activation (16 warps per SM to issue
+// them, issue active 46 %), and the pair's exchange between layers; the next
+// weights arrive (cp.async.bulk) under it.  Measured against a kernel per
+// layer with activations in HBM and 4 warps per SM (B200): prediction of 300,007
+// rows 2,005 -> 593 us, a training step on 8,192 rows 753 -> 105 us
+// (net_kernel 46, dw_kernel 34, adam_kernel 7).  Swizzled operand tiles were
+// measured too (no faster: the products are not the bound; their strided
+// writes to the peer cost 10 %).
 //
 // Every product is one elected thread issuing tcgen05.mma of BF16 operands
-// in shared memory (canonical K-major layout, e2d_tc.cuh) into an FP32 TMEM
-// accumulator, committed to an mbarrier that the CTA waits on with a bounded
-// spin; a wait that runs out sets the error word and the kernel returns
-// after freeing its TMEM.  One CTA of 128 threads per SM, persistent over
-// tiles of 128 rows (a row is a TMEM lane, a thread its epilogue).
+// in shared memory (e2d_tc.cuh) into an FP32 TMEM accumulator, committed to an
+// mbarrier that is waited on with a bounded spin; a wait that runs out sets the
+// error word, the remaining products are skipped and the TMEM is freed.
+// Activations, deltas and weights live in global memory in the canonical
+// operand layout (tiles of 128 rows), so that a tile, half or chunk of one is
+// a plain bulk copy, and the weight gradients read the same tiles as MN-major
+// operands: no transposed copies.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <vector>
@@ -32,7 +48,9 @@ namespace {
 
 constexpr int DF = 16, DH = 256, DO = 16, DO_USED = 4, DNL = 4;  // features, width, outputs (padded), hidden layers
 constexpr int NLAYER = DNL + 1;
-constexpr int TILE = 128;          // rows per tile (UMMA M), threads per CTA
+constexpr int TILE = 128;          // rows per tile (UMMA M)
+constexpr int HALF = DH / 2;       // columns of a layer per CTA of a pair
+constexpr int NT = 512;            // threads of net_kernel: 4 warps per 32 TMEM lanes
 constexpr int RC = 64;             // rows per chunk of the weight-gradient product
 constexpr uint32_t WAIT_ITERS = 1u << 22;
 
@@ -40,37 +58,28 @@ __host__ __device__ constexpr int layer_in(int l) { return l == 0 ? DF : DH; }
 __host__ __device__ constexpr int layer_out(int l) { return l == DNL ? DO : DH; }
 // flat parameter vector: W_l [out][in] then b_l [out], layers 0..4
 __host__ __device__ constexpr int w_off(int l) {
-  return l == 0 ? 0 : w_off(l - 1) + layer_out(l - 1) * layer_in(l - 1) + layer_out(l - 1);
+  return l == 0 ? 0 : DH * DF + DH + (l - 1) * (DH * DH + DH) - (l == NLAYER ? (DH - DO) * (DH + 1) : 0);
 }
 __host__ __device__ constexpr int b_off(int l) { return w_off(l) + layer_out(l) * layer_in(l); }
 constexpr int NPARAM = w_off(NLAYER);
-
-enum Epi { FWD_GELU = 0, FWD_LINEAR = 1, BWD_GELU = 2 };
+static_assert(NPARAM == w_off(DNL) + DO * DH + DO, "parameter layout");
 
 __device__ __forceinline__ uint16_t f2bf(float x) { return __bfloat16_as_ushort(__float2bfloat16_rn(x)); }
 __device__ __forceinline__ float bf2f(uint16_t b) { return __uint_as_float(uint32_t(b) << 16); }
 
-// GELU, tanh form, and its derivative.
-__device__ __forceinline__ float gelu(float z) {
-  const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-  return 0.5f * z * (1.0f + tanhf(u));
-}
-__device__ __forceinline__ float gelu_prime(float z) {
+// GELU, tanh form, and its derivative (null: not wanted), from one tanh.
+__device__ __forceinline__ float gelu(float z, float* prime) {
   const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
   const float t = tanhf(u);
-  return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 0.134145f * z * z);
+  if (prime) *prime = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 0.134145f * z * z);
+  return 0.5f * z * (1.0f + t);
 }
 
-// Row-major BF16 [rows][K] (global) -> canonical K-major tile (shared), 16
-// bytes (8 values of one row) at a time; rows at or past `valid` are zero.
-__device__ void stage_tile(uint8_t* dst, const uint16_t* src, int rows, int K, int valid) {
-  const int per_row = K / 8;
-  for (int q = threadIdx.x; q < rows * per_row; q += TILE) {
-    const int r = q / per_row, c = (q % per_row) * 8;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < valid) v = *reinterpret_cast<const uint4*>(src + size_t(r) * K + c);
-    *reinterpret_cast<uint4*>(dst + tc::kmaj_off(r, c, K)) = v;
-  }
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  uint32_t k[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) k[q] = uint32_t(f2bf(v[2 * q])) | (uint32_t(f2bf(v[2 * q + 1])) << 16);
+  return make_uint4(k[0], k[1], k[2], k[3]);
 }
 
 __device__ __forceinline__ void cta_sync_async() {
@@ -83,277 +92,510 @@ __device__ __forceinline__ void cta_sync_async() {
 // Commit (thread 0) and bounded wait of every thread; CTA-uniform result.
 __device__ __forceinline__ bool complete(uint64_t* bar, uint32_t& phase) {
   if (threadIdx.x == 0) tc::mma_commit(bar);
-  __syncwarp();
-  const bool ok = tc::mbar_wait(bar, phase, WAIT_ITERS);
+  const bool ok = tc::mbar_wait_warp(bar, phase, WAIT_ITERS);
   phase ^= 1u;
   tc::fence_after_sync();
   return __syncthreads_and(ok) != 0;
 }
 
-__host__ __device__ inline uint32_t tmem_cols(int n) {
-  uint32_t c = 32;
-  while (c < uint32_t(n)) c <<= 1;
-  return c;
+// Tiles of 128 rows (activations, deltas, features) are column-chunk tiles
+// (e2d_tc.cuh): any range of columns is contiguous, so a CTA's half of a tile
+// goes to global memory, and a piece of one to the weight gradients, as one
+// bulk copy, and a warp's 32 rows of a chunk are 512 bytes on end.  Weights
+// are K-major by row group: a half of the rows is contiguous.
+constexpr int CHUNK = TILE * 16;
+__device__ __forceinline__ uint32_t tile_off(int r, int k) {  // byte of element (r, k)
+  return uint32_t((k >> 3) * CHUNK + r * 16 + (k & 7) * 2);
 }
 
-// D[tile rows][N] = A[tile rows][K] B[N][K]^T with the epilogue EPI; B stays
-// in shared memory for all of the CTA's tiles.  K and N: multiples of 16, at
-// most 256.
-template <int EPI>
-__global__ void __launch_bounds__(TILE, 1) dense_kernel(const uint16_t* __restrict__ A, int K,
-                                                        const uint16_t* __restrict__ Bw, int N,
-                                                        const float* __restrict__ bias, int n,
-                                                        float* __restrict__ Zout, uint16_t* __restrict__ Hout,
-                                                        const float* __restrict__ Zp, float* __restrict__ Yout,
-                                                        int* err) {
-  extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ uint64_t bar;
-  __shared__ uint32_t taddr;
-  uint8_t* Bs = sm;                      // [N][K]
-  uint8_t* As = sm + size_t(N) * K * 2;  // [TILE][K]
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t ncols = tmem_cols(N);
-  stage_tile(Bs, Bw, N, K, N);
-  if (tid == 0) tc::mbar_init(&bar, 1);
-  if (warp == 0) tc::tmem_alloc(&taddr, ncols);
+// D[128][N] = A[128][K] B[N][K]^T, one thread: A a tile, B weights.
+__device__ __forceinline__ void product(uint32_t d, const uint8_t* A, const uint8_t* Bm, int K, int N) {
+  const uint32_t id = tc::idesc_bf16(TILE, N), a0 = tc::smem_addr(A), b0 = tc::smem_addr(Bm);
+  for (int t = 0; t < K / 16; ++t)
+    tc::mma_bf16(d, tc::smem_desc(a0 + 2 * CHUNK * t, CHUNK, 128), tc::smem_desc(b0 + 256 * t, 128, K * 16), id,
+                 t > 0 ? 1u : 0u);
+}
+
+// Four floats of a caller's array: one 16-byte access where its base is
+// 16-byte aligned (vec), else four.
+__device__ __forceinline__ float4 ld4(const float* p, int vec) {
+  return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
+struct NetArgs {
+  const float *X, *T;         // [*][16], [*][4]
+  int vec;                    // X, T and Y are 16-byte aligned
+  const int* idx;             // rows of the pass (null: 0 .. n-1)
+  int n;
+  float inv_n;
+  const uint16_t *wk, *wt;    // BF16 weights and transposes, canonical tiles at the parameter offsets
+  const float* p;             // FP32 parameters (biases)
+  float* Y;                   // [n][4] (forward)
+  uint16_t *xb, *dy;          // tiles [128][16] (train)
+  uint16_t *act[DNL], *dz[DNL];  // tiles [128][256] (train)
+  float* gp;                  // GELU' of the CTA's current tile, [CTA][4][128 x 128] (train)
+  double* lpart;              // loss sums, [clusters] (train)
+  int* err;
+};
+
+struct NetSmem {
+  uint8_t A[2][TILE * DH * 2];    // activations / deltas, [128][256]
+  uint8_t W[HALF * DH * 2];       // this CTA's half of a hidden layer's weights or transpose
+  uint8_t W0[HALF * DF * 2], W4[DO * DH * 2], W4T[HALF * DO * 2];
+  uint8_t X[TILE * DF * 2], dY[TILE * DO * 2];
+  float b[DNL][HALF], b4[DO];
+  double lw[4];
+  uint64_t bar, wbar;
+  uint32_t taddr;
+};
+
+template <bool TRAIN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) net_kernel(const __grid_constant__ NetArgs a) {
+  extern __shared__ __align__(1024) uint8_t smraw[];
+  NetSmem& s = *reinterpret_cast<NetSmem*>(smraw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const uint32_t rank = tc::cluster_rank();
+  const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
+  const int ntiles = (a.n + TILE - 1) / TILE;
+  // constant operands (16 bytes a thread) and biases
+  auto copy = [&](uint8_t* dst, const uint16_t* src, int bytes) {
+    for (int q = tid; q < bytes / 16; q += NT) reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<const uint4*>(src)[q];
+  };
+  copy(s.W0, a.wk + w_off(0) + rank * HALF * DF, HALF * DF * 2);
+  copy(s.W4, a.wk + w_off(DNL), DO * DH * 2);
+  if (TRAIN) copy(s.W4T, a.wt + w_off(DNL) + rank * HALF * DO, HALF * DO * 2);
+  if (tid < HALF)
+    for (int l = 0; l < DNL; ++l) s.b[l][tid] = a.p[b_off(l) + rank * HALF + tid];
+  if (tid < DO) s.b4[tid] = a.p[b_off(DNL) + tid];
+  if (tid == 0) {
+    tc::mbar_init(&s.bar, 1);
+    tc::mbar_init(&s.wbar, 1);
+  }
+  if (warp == 0) tc::tmem_alloc(&s.taddr, 256);
   cta_sync_async();
-  const uint32_t tm = taddr;
-  const uint32_t lane_base = uint32_t(32 * warp) << 16;
-  const uint32_t id = tc::idesc_bf16(TILE, N);
-  uint32_t phase = 0;
-  const int ntiles = (n + TILE - 1) / TILE;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int r0 = tile * TILE;
-    stage_tile(As, A + size_t(r0) * K, TILE, K, n - r0);
-    cta_sync_async();
+  tc::cluster_sync();  // the peer runs: its shared memory may be written
+  const uint32_t tm = s.taddr, td = tm, ty = tm + HALF;  // hidden products, outputs
+  // this thread's TMEM lane (row of the tile) and 32 of the CTA's 128 columns
+  const int row = 32 * (warp & 3) + lane, cg = warp >> 2;
+  const uint32_t lane_base = uint32_t(32 * (warp & 3)) << 16;
+  const uint32_t roff = tile_off(row, 0);
+  const uint32_t peer = rank ^ 1u;
+  const uint32_t pA[2] = {tc::peer_addr(tc::smem_addr(s.A[0]), peer), tc::peer_addr(tc::smem_addr(s.A[1]), peer)};
+  float4* gp = TRAIN ? reinterpret_cast<float4*>(a.gp) + size_t(blockIdx.x) * (DNL * TILE * HALF / 4) : nullptr;
+  uint32_t phase = 0, wphase = 0;
+  int wissued = 0, wwaited = 0;
+  bool ok = true;
+  double lsum = 0.0;
+  // one hidden layer's weights (its transpose for the deltas) into s.W
+  auto load_w = [&](const uint16_t* src) {
+    ++wissued;
     if (tid == 0) {
-      const uint32_t a0 = tc::smem_addr(As), b0 = tc::smem_addr(Bs);
-      for (int t = 0; t < K / 16; ++t)
-        tc::mma_bf16(tm, tc::smem_desc(a0 + 256 * t, 128, K * 16), tc::smem_desc(b0 + 256 * t, 128, K * 16), id,
-                     t > 0 ? 1u : 0u);
+      tc::mbar_expect_tx(&s.wbar, HALF * DH * 2);
+      for (int q = 0; q < 4; ++q)
+        tc::bulk_load(s.W + q * (HALF * DH / 2), src + rank * HALF * DH + q * (HALF * DH / 4), HALF * DH / 2, &s.wbar);
     }
-    if (!complete(&bar, phase)) {
-      if (tid == 0) atomicExch(err, 1);
-      break;
+  };
+  auto wait_w = [&]() {
+    const bool got = tc::mbar_wait_warp(&s.wbar, wphase, WAIT_ITERS);
+    wphase ^= 1u;
+    ++wwaited;
+    ok = __syncthreads_and(got && ok) != 0;
+  };
+  // both CTAs' halves of the next operand are in buffer nxt; this CTA's half
+  // goes to global memory too (out not null)
+  auto pair_sync = [&](int nxt, uint16_t* out) {
+    asm volatile("fence.proxy.async;" ::: "memory");
+    tc::fence_before_sync();
+    tc::cluster_sync();
+    tc::fence_after_sync();
+    if (tid == 0) {
+      asm volatile("fence.proxy.async;" ::: "memory");
+      if (out) tc::bulk_store(out + rank * HALF * TILE, s.A[nxt] + rank * HALF * TILE * 2, HALF * TILE * 2);
     }
-    const int row = r0 + tid;
-    const bool valid = row < n;
-    for (int c0 = 0; c0 < N; c0 += 16) {
-      float v[16];
-      tc::tmem_ld16(tm + lane_base + uint32_t(c0), v);
-      if (!valid) continue;
-      if (EPI == FWD_GELU || EPI == FWD_LINEAR) {
+  };
+  // 16 values of this thread's row, columns rank * 128 + 32 cg + 16 h of a
+  // layer, as BF16 into buffer nxt, the peer's too (both)
+  auto put16 = [&](const float* v, int h, int nxt, bool both) {
+    const int c = rank * (HALF / 8) + 4 * cg + 2 * h;  // chunk of 8 columns
 #pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] += bias[c0 + q];
+    for (int q = 0; q < 2; ++q) {
+      const uint4 k = pack8(v + 8 * q);
+      const uint32_t off = roff + (c + q) * CHUNK;
+      *reinterpret_cast<uint4*>(s.A[nxt] + off) = k;
+      if (both) tc::st_peer(pA[nxt] + off, k);
+    }
+  };
+  if (cluster < ntiles) load_w(a.wk + w_off(1));
+  for (int tile = cluster; tile < ntiles; tile += nclusters) {
+    const int grow = tile * TILE + row;
+    const bool valid = grow < a.n, more = tile + nclusters < ntiles;
+    if (tid < 2 * TILE) {  // X: 8 features a thread
+      const int r = tid & (TILE - 1), c = tid >> 7, g = tile * TILE + r;
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (g < a.n) {
+        const float* x = a.X + size_t(a.idx ? a.idx[g] : g) * DF + 8 * c;
+        const float4 x0 = ld4(x, a.vec), x1 = ld4(x + 4, a.vec);
+        v[0] = x0.x; v[1] = x0.y; v[2] = x0.z; v[3] = x0.w; v[4] = x1.x; v[5] = x1.y; v[6] = x1.z; v[7] = x1.w;
       }
-      if (EPI == FWD_LINEAR) {
-        float4* y = reinterpret_cast<float4*>(Yout + size_t(row) * N + c0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) y[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        continue;
+      const uint4 k = pack8(v);
+      const uint32_t off = tile_off(r, 8 * c);
+      *reinterpret_cast<uint4*>(s.X + off) = k;
+      if (TRAIN && rank == 0)
+        *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.xb) + size_t(tile) * (TILE * DF * 2) + off) = k;
+    }
+    cta_sync_async();
+    // ---- hidden layers: H_l = gelu(A W_l^T + b_l) --------------------------
+    for (int l = 0; l < DNL; ++l) {
+      if (l > 0) wait_w();
+      if (ok) {
+        if (tid == 0) {
+          if (l == 0) product(td, s.X, s.W0, DF, HALF);
+          else product(td, s.A[(l - 1) & 1], s.W, DH, HALF);
+          if (TRAIN) tc::bulk_store_read<1>();  // the buffer written next has reached global memory
+        }
+        ok = complete(&s.bar, phase);
       }
-      if (EPI == FWD_GELU) {
-        float4* z = reinterpret_cast<float4*>(Zout + size_t(row) * N + c0);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) z[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-#pragma unroll
-        for (int q = 0; q < 16; ++q) v[q] = gelu(v[q]);
-      } else {  // BWD_GELU
-        const float4* zp = reinterpret_cast<const float4*>(Zp + size_t(row) * N + c0);
+      if (l > 0) {  // the weights are read: the next ones arrive under the epilogue
+        if (l < DNL - 1) load_w(a.wk + w_off(l + 1));
+        else if (TRAIN) load_w(a.wt + w_off(DNL - 1));
+        else if (more) load_w(a.wk + w_off(1));
+      }
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        float v[16], g[16];
+        tc::tmem_ld16(td + lane_base + uint32_t(32 * cg + 16 * h), v);
+        const float4* b = reinterpret_cast<const float4*>(&s.b[l][32 * cg + 16 * h]);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          const float4 z = zp[q];
-          v[4 * q] *= gelu_prime(z.x); v[4 * q + 1] *= gelu_prime(z.y);
-          v[4 * q + 2] *= gelu_prime(z.z); v[4 * q + 3] *= gelu_prime(z.w);
+          const float4 bq = b[q];
+          v[4 * q] += bq.x; v[4 * q + 1] += bq.y; v[4 * q + 2] += bq.z; v[4 * q + 3] += bq.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const float y = gelu(v[q], TRAIN ? &g[q] : nullptr);
+          v[q] = !TRAIN || valid ? y : 0.0f;  // rows past the last stay zero in the gradients
+        }
+        if (TRAIN)
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            gp[(((l * 4 + cg) * 2 + h) * 4 + q) * TILE + row] =
+                make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
+        put16(v, h, l & 1, true);
+      }
+      pair_sync(l & 1, TRAIN ? a.act[l] + size_t(tile) * (TILE * DH) : nullptr);
+    }
+    // ---- outputs -------------------------------------------------------------
+    if (ok && (TRAIN || rank == 0)) {
+      if (tid == 0) product(ty, s.A[(DNL - 1) & 1], s.W4, DH, DO);
+      ok = complete(&s.bar, phase);
+    }
+    if (!TRAIN) {
+      if (rank == 0 && warp < 4) {
+        float y[16];
+        tc::tmem_ld16(ty + lane_base, y);
+        float* o = a.Y + size_t(grow) * DO_USED;
+        if (valid && a.vec)
+          *reinterpret_cast<float4*>(o) = make_float4(y[0] + s.b4[0], y[1] + s.b4[1], y[2] + s.b4[2], y[3] + s.b4[3]);
+        else if (valid)
+#pragma unroll
+          for (int q = 0; q < DO_USED; ++q) o[q] = y[q] + s.b4[q];
+      }
+      tc::fence_before_sync();
+      continue;
+    }
+    // ---- loss and the output deltas dY = bf16(2 (y - t) / n) -------------------
+    if (warp < 4) {
+      float y[16], d[16];
+      tc::tmem_ld16(ty + lane_base, y);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) d[q] = 0.0f;
+      if (valid) {
+        const float4 t = ld4(a.T + size_t(a.idx ? a.idx[grow] : grow) * DO_USED, a.vec);
+        const float tq[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int q = 0; q < DO_USED; ++q) {
+          const float e = (y[q] + s.b4[q]) - tq[q];
+          lsum += double(e) * double(e);
+          d[q] = 2.0f * e * a.inv_n;
         }
       }
-      uint32_t pk[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) pk[q] = uint32_t(f2bf(v[2 * q])) | (uint32_t(f2bf(v[2 * q + 1])) << 16);
-      uint4* h = reinterpret_cast<uint4*>(Hout + size_t(row) * N + c0);
-      h[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
-      h[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+      for (int q = 0; q < 2; ++q) {
+        const uint4 k = pack8(d + 8 * q);
+        const uint32_t off = tile_off(row, 8 * q);
+        *reinterpret_cast<uint4*>(s.dY + off) = k;
+        if (rank == 0)
+          *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(a.dy) + size_t(tile) * (TILE * DO * 2) + off) = k;
+      }
     }
-  }
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  if (warp == 0) tc::tmem_dealloc(tm, ncols);
-}
-
-// Row-major BF16 [rows][F] (global) -> the transposed canonical tile
-// [F][RC] (shared; K = rows): element (f, r) at kmaj_off(f, r, RC).
-__device__ void stage_transposed(uint8_t* dst, const uint16_t* src, int rows, int F, int valid) {
-  const int per_row = F / 8;
-  for (int q = threadIdx.x; q < rows * per_row; q += TILE) {
-    const int r = q / per_row, f0 = (q % per_row) * 8;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (r < valid) v = *reinterpret_cast<const uint4*>(src + size_t(r) * F + f0);
-    const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
-#pragma unroll
-    for (int k = 0; k < 8; ++k) *reinterpret_cast<uint16_t*>(dst + tc::kmaj_off(f0 + k, r, RC)) = e[k];
-  }
-}
-
-// slot[blockIdx][256][N2] = P^T Q over the CTA's rows [r0, r1): P [n][256],
-// Q [n][N2] row-major BF16, N2 16 or 256; the two 128-row halves of P^T
-// accumulate in TMEM columns [0, N2) and [N2, 2 N2).
-__global__ void __launch_bounds__(TILE, 1) dw_kernel(const uint16_t* __restrict__ P, const uint16_t* __restrict__ Q,
-                                                     int N2, int n, int rows_per_cta, float* __restrict__ slots,
-                                                     int* err) {
-  extern __shared__ __align__(1024) uint8_t sm[];
-  __shared__ uint64_t bar;
-  __shared__ uint32_t taddr;
-  uint8_t* Ps = sm;                      // [256][RC]
-  uint8_t* Qs = sm + size_t(DH) * RC * 2;  // [N2][RC]
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const uint32_t ncols = tmem_cols(2 * N2);
-  if (tid == 0) tc::mbar_init(&bar, 1);
-  if (warp == 0) tc::tmem_alloc(&taddr, ncols);
-  cta_sync_async();
-  const uint32_t tm = taddr;
-  const uint32_t lane_base = uint32_t(32 * warp) << 16;
-  const uint32_t id = tc::idesc_bf16(TILE, N2);
-  const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
-  uint32_t phase = 0;
-  bool ok = true, any = false;
-  for (int c = r0; c < r1 && ok; c += RC) {
-    stage_transposed(Ps, P + size_t(c) * DH, RC, DH, r1 - c);
-    stage_transposed(Qs, Q + size_t(c) * N2, RC, N2, r1 - c);
     cta_sync_async();
-    if (tid == 0) {
-      const uint32_t p0 = tc::smem_addr(Ps), q0 = tc::smem_addr(Qs);
-      for (int h = 0; h < 2; ++h)
-        for (int t = 0; t < RC / 16; ++t)
-          tc::mma_bf16(tm + uint32_t(h * N2), tc::smem_desc(p0 + h * (TILE * RC * 2) + 256 * t, 128, RC * 16),
-                       tc::smem_desc(q0 + 256 * t, 128, RC * 16), id, (any || t > 0) ? 1u : 0u);
-    }
-    any = true;
-    ok = complete(&bar, phase);
-  }
-  if (!ok) {
-    if (tid == 0) atomicExch(err, 1);
-  } else {
-    float* out = slots + size_t(blockIdx.x) * DH * N2;
-    for (int h = 0; h < 2; ++h) {
-      const int f = h * TILE + tid;
-      for (int c0 = 0; c0 < N2; c0 += 16) {
+    // ---- hidden deltas: dZ_l = (dZ_{l+1} W_{l+1}) * gelu'(Z_l) -----------------
+    for (int l = DNL - 1; l >= 0; --l) {
+      const bool top = l == DNL - 1;
+      if (!top) wait_w();
+      if (ok) {
+        if (tid == 0) {
+          if (top) product(td, s.dY, s.W4T, DO, HALF);
+          else product(td, s.A[l & 1], s.W, DH, HALF);
+          tc::bulk_store_read<1>();
+        }
+        ok = complete(&s.bar, phase);
+      }
+      if (!top) {
+        if (l > 0) load_w(a.wt + w_off(l));
+        else if (more) load_w(a.wk + w_off(1));
+      }
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
         float v[16];
-        tc::tmem_ld16(tm + lane_base + uint32_t(h * N2 + c0), v);
+        tc::tmem_ld16(td + lane_base + uint32_t(32 * cg + 16 * h), v);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) out[size_t(f) * N2 + c0 + q] = any ? v[q] : 0.0f;
+        for (int q = 0; q < 4; ++q) {
+          const float4 g = gp[(((l * 4 + cg) * 2 + h) * 4 + q) * TILE + row];
+          v[4 * q] *= g.x; v[4 * q + 1] *= g.y; v[4 * q + 2] *= g.z; v[4 * q + 3] *= g.w;
+        }
+#pragma unroll
+        for (int q = 0; q < 16; ++q) v[q] = valid ? v[q] : 0.0f;
+        // the next product (layer l - 1) reads buffer (l - 1) & 1
+        put16(v, h, (l - 1) & 1, l > 0);
+      }
+      pair_sync((l - 1) & 1, a.dz[l] + size_t(tile) * (TILE * DH));
+    }
+  }
+  if (TRAIN && rank == 0 && warp < 4) {
+    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
+    if (lane == 0) s.lw[warp] = lsum;
+  }
+  if (wissued > wwaited) tc::mbar_wait(&s.wbar, wphase, WAIT_ITERS);  // no copy outlives the CTA
+  if (TRAIN && tid == 0) tc::bulk_store_done();
+  if (!ok && tid == 0) atomicExch(a.err, 1);
+  tc::fence_before_sync();
+  tc::cluster_sync();
+  tc::fence_after_sync();
+  if (TRAIN && rank == 0 && tid == 0) a.lpart[cluster] = ((s.lw[0] + s.lw[1]) + s.lw[2]) + s.lw[3];
+  if (warp == 0) tc::tmem_dealloc(tm, 256);
+}
+
+// ---- weight and bias gradients -----------------------------------------------
+// dW_l = sum over rows of dZ_l^T A_l, the rows in groups of `rows` (a multiple
+// of 64): a group is accumulated by the tensor core, the groups are added in
+// order in FP32 registers, so the sum is the same whichever SM forms it.  One
+// CTA per 128 x DWN piece of a layer's gradient walks all groups: one warp
+// brings the tiles' columns of both operands (one bulk copy each, a ring of
+// DWS stages), DWI warps issue the products of a group each in turn (a product
+// of 64 rows is four small MMAs, so one thread's issue rate bounds it: 74 us
+// with one such warp, 34 with four, 8,192 rows), four warps add.  Before,
+// every group's gradient went to a slot and the slots were summed: 33 MB a
+// layer each way, 430 us a step.
+constexpr int DWN = 32;                            // columns of a piece
+constexpr int DWS = 5;                             // stages
+constexpr int DWB = 256 / DWN;                             // accumulators: a group's product, read and release overlap the others'
+constexpr int DW_P = TILE * HALF * 2, DW_Q = TILE * DWN * 2;  // bytes of a tile's operands
+constexpr int DW_HID = (DNL - 1) * 2 * (DH / DWN);  // pieces of the 256 x 256 layers
+constexpr int DW_ITEMS = DW_HID + 4;               // and two halves each of the first and the output layer
+constexpr int BCOLS = 16;                          // columns of a bias piece: two threads a row, 144 groups at a time
+constexpr int DW_BIAS = DNL * (DH / BCOLS) + 1;    // bias pieces of the hidden layers, and the outputs'
+constexpr int DWI = 4;                             // warps that issue products, a group each in turn
+constexpr int DW_THREADS = 32 * (4 + 1 + DWI);
+static_assert(DWB * DWN == 256, "TMEM columns: a power of two, at least 32");
+static_assert(DF == 16 && DO == 16, "the narrow layers are one piece of 16 columns");
+
+struct DwArgs {
+  const uint16_t *xb, *dy;
+  const uint16_t *act[DNL], *dz[DNL];
+  int n, rows, brows;  // rows per group of the products, of the bias sums
+  float* g;
+  int* err;
+};
+struct DwSmem {
+  uint8_t P[DWS][DW_P], Q[DWS][DW_Q];
+  uint64_t full[DWS], empty[DWS], dfull[DWB], dempty[DWB];
+  uint32_t taddr;
+  int failed;
+};
+constexpr int BIAS_MAX_GROUPS = 512;  // at most one group per SM
+static_assert(DO == BCOLS && sizeof(DwSmem) >= BIAS_MAX_GROUPS * BCOLS * 4, "bias partial sums fit");
+
+// db_l: the rows in groups of brows, each summed in row order, then the
+// groups in order.  A thread sums 8 columns (16 bytes a row).
+__device__ void bias_piece(const DwArgs& a, int item, float* part) {
+  const bool hid = item < DNL * (DH / BCOLS);
+  const int l = hid ? item / (DH / BCOLS) : DNL, c0 = hid ? BCOLS * (item % (DH / BCOLS)) : 0;
+  const int sub = threadIdx.x / (BCOLS / 8), c = threadIdx.x % (BCOLS / 8), nsub = DW_THREADS / (BCOLS / 8);
+  const uint8_t* D = reinterpret_cast<const uint8_t*>(hid ? a.dz[l] : a.dy) + tile_off(0, c0 + 8 * c);
+  const size_t tile = TILE * 2 * (hid ? DH : DO);
+  const int groups = (a.n + a.brows - 1) / a.brows;
+  for (int k = sub; k < groups; k += nsub) {
+    const int r0 = k * a.brows, r1 = min(a.n, r0 + a.brows);
+    float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 16
+    for (int r = r0; r < r1; ++r) {
+      const uint4 v = *reinterpret_cast<const uint4*>(D + (r >> 7) * tile + tile_off(r & (TILE - 1), 0));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        t[2 * e] += bf2f(uint16_t(w[e]));
+        t[2 * e + 1] += bf2f(uint16_t(w[e] >> 16));
       }
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) part[k * BCOLS + 8 * c + e] = t[e];
   }
+  __syncthreads();
+  if (threadIdx.x < BCOLS) {
+    float t = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < groups; ++k) t += part[k * BCOLS + threadIdx.x];
+    a.g[b_off(l) + c0 + threadIdx.x] = hid || threadIdx.x < DO_USED ? t : 0.0f;
+  }
+}
+
+__global__ void __launch_bounds__(DW_THREADS, 1) dw_kernel(const __grid_constant__ DwArgs a) {
+  extern __shared__ __align__(1024) uint8_t smraw[];
+  DwSmem& s = *reinterpret_cast<DwSmem*>(smraw);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, item = blockIdx.x;
+  if (item >= DW_ITEMS) {
+    bias_piece(a, item - DW_ITEMS, reinterpret_cast<float*>(smraw));
+    return;
+  }
+  const bool hid = item < DW_HID, last = item >= DW_HID + 2;
+  const int l = hid ? 1 + item / (2 * (DH / DWN)) : (last ? DNL : 0);
+  const int half = hid ? (item / (DH / DWN)) & 1 : item & 1, nt = hid ? item % (DH / DWN) : 0;
+  const int ncol = hid ? DWN : 16;
+  const uint32_t qbytes = TILE * 2 * ncol;
+  const uint8_t* P = reinterpret_cast<const uint8_t*>(last ? a.act[DNL - 1] : a.dz[l]) + half * DW_P;
+  const uint8_t* Q = reinterpret_cast<const uint8_t*>(hid ? a.act[l - 1] : (last ? a.dy : a.xb)) + nt * DW_Q;
+  const size_t qtile = hid ? TILE * DH * 2 : qbytes;  // bytes of a tile of Q's array
+  if (tid == 0) {
+    for (int k = 0; k < DWS; ++k) {
+      tc::mbar_init(&s.full[k], 1);
+      tc::mbar_init(&s.empty[k], 2);  // the tile's two chunks of 64 rows
+    }
+    for (int k = 0; k < DWB; ++k) {
+      tc::mbar_init(&s.dfull[k], 1);
+      tc::mbar_init(&s.dempty[k], 4);
+    }
+    s.failed = 0;
+  }
+  if (warp == 0) tc::tmem_alloc(&s.taddr, DWB * DWN);
+  cta_sync_async();
+  const uint32_t tm = s.taddr;
+  const int nchunk = (a.n + RC - 1) / RC, per = a.rows / RC, ngroup = (nchunk + per - 1) / per;
+  float acc[DWN];
+#pragma unroll
+  for (int q = 0; q < DWN; ++q) acc[q] = 0.0f;
+  bool ok = true;
+  const int ntiles = (a.n + TILE - 1) / TILE;
+  if (warp == 4) {  // copies
+    int k = 0;
+    for (; k < ntiles; ++k) {
+      const int st = k % DWS;
+      if (k >= DWS) ok = tc::mbar_wait_warp(&s.empty[st], uint32_t(k / DWS - 1) & 1u, WAIT_ITERS);
+      if (!ok) break;
+      if (lane == 0) {
+        tc::mbar_expect_tx(&s.full[st], DW_P + qbytes);
+        tc::bulk_load(s.P[st], P + size_t(k) * (TILE * DH * 2), DW_P, &s.full[st]);
+        tc::bulk_load(s.Q[st], Q + k * qtile, qbytes, &s.full[st]);
+      }
+      __syncwarp();
+    }
+    for (int j = max(0, k - DWS); j < k; ++j) {  // no product and, stopped early, no copy outlives the CTA
+      if (ok) ok = tc::mbar_wait_warp(&s.empty[j % DWS], uint32_t(j / DWS) & 1u, WAIT_ITERS);
+      else tc::mbar_wait(&s.full[j % DWS], uint32_t(j / DWS) & 1u, WAIT_ITERS);
+    }
+  } else if (warp > 4) {  // products: group after group, DWI warps in turn, 64 rows at a time
+    if (lane == 0) {
+      const uint32_t id = tc::idesc_bf16_t(TILE, ncol);
+      for (int grp = warp - 5; grp < ngroup && ok; grp += DWI) {
+        const int buf = grp % DWB, k1 = min(nchunk, (grp + 1) * per);
+        if (grp >= DWB) ok = tc::mbar_wait(&s.dempty[buf], uint32_t(grp / DWB - 1) & 1u, WAIT_ITERS);
+        for (int k = grp * per; k < k1; ++k) {
+          const int tile = k >> 1, st = tile % DWS;
+          ok = ok && tc::mbar_wait(&s.full[st], uint32_t(tile / DWS) & 1u, WAIT_ITERS);
+          if (!ok) break;
+          tc::fence_after_sync();
+          const uint32_t p0 = tc::smem_addr(s.P[st]) + (k & 1) * (CHUNK / 2);
+          const uint32_t q0 = tc::smem_addr(s.Q[st]) + (k & 1) * (CHUNK / 2);
+#pragma unroll
+          for (int t = 0; t < RC / 16; ++t)  // 16 rows: two row groups
+            tc::mma_bf16(tm + buf * DWN, tc::smem_desc(p0 + 256 * t, 128, CHUNK), tc::smem_desc(q0 + 256 * t, 128, CHUNK),
+                         id, (k > grp * per || t > 0) ? 1u : 0u);
+          if (k == k1 - 1) tc::mma_commit(&s.dfull[buf]);
+          tc::mma_commit(&s.empty[st]);
+          if (k == nchunk - 1 && !(k & 1)) tc::mma_commit(&s.empty[st]);  // the last tile's missing half
+        }
+      }
+    }
+    ok = __shfl_sync(0xffffffffu, int(ok), 0) != 0;
+  } else {  // sums: TMEM lane = row of the piece
+    const uint32_t lane_base = uint32_t(32 * warp) << 16;
+    for (int grp = 0; grp < ngroup && ok; ++grp) {
+      const int buf = grp % DWB;
+      ok = tc::mbar_wait_warp(&s.dfull[buf], uint32_t(grp / DWB) & 1u, WAIT_ITERS);
+      if (!ok) break;
+      tc::fence_after_sync();
+      float v[DWN];  // (columns past a narrow piece's 16 are read and not used)
+      tc::tmem_ld32(tm + lane_base + uint32_t(buf * DWN), v);
+#pragma unroll
+      for (int q = 0; q < DWN; ++q) acc[q] += v[q];
+      tc::fence_before_sync();
+      if (lane == 0) tc::mbar_arrive(&s.dempty[buf]);
+    }
+    const int f = half * HALF + 32 * warp + lane;
+    if (last) {  // W5 [16][256]: rows past the used outputs stay 0
+#pragma unroll
+      for (int q = 0; q < DO; ++q) a.g[w_off(DNL) + q * DH + f] = q < DO_USED ? acc[q] : 0.0f;
+    } else {
+      float4* o = reinterpret_cast<float4*>(a.g + w_off(l) + f * layer_in(l) + nt * DWN);
+#pragma unroll
+      for (int q = 0; q < DWN / 4; ++q)
+        if (4 * q < ncol) o[q] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+    }
+  }
+  if (!ok && lane == 0) atomicExch(a.err, 1);
   tc::fence_before_sync();
   __syncthreads();
   tc::fence_after_sync();
-  if (warp == 0) tc::tmem_dealloc(tm, ncols);
+  if (warp == 0) tc::tmem_dealloc(tm, DWB * DWN);
 }
 
-// The CTAs' slots summed in CTA order into the gradient of W_l: slot layout
-// [256][N2]; transpose = the slots hold W_l^T (the output layer).
-__global__ void dw_reduce_kernel(const float* __restrict__ slots, int nslot, int N2, float* __restrict__ g,
-                                 int woff, int transpose) {
-  const int total = DH * N2;
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < total; q += gridDim.x * blockDim.x) {
-    float t = 0.0f;
-    for (int c = 0; c < nslot; ++c) t += slots[size_t(c) * total + q];
-    const int f = q / N2, k = q % N2;
-    if (transpose) {
-      g[woff + k * DH + f] = k < DO_USED ? t : 0.0f;  // W5 [16][256]: rows past the used outputs stay 0
-    } else {
-      g[woff + q] = t;
-    }
-  }
+// The BF16 copies of weight q: of W_l [out][in] and, past the first layer, of
+// its transpose [in][out].
+__device__ __forceinline__ void put_weight(int q, float x, uint16_t* wk, uint16_t* wt) {
+  int l = 0;
+  while (l < NLAYER - 1 && q >= w_off(l + 1)) ++l;
+  const int rel = q - w_off(l);
+  if (rel >= layer_out(l) * layer_in(l)) return;  // a bias
+  const int o = rel / layer_in(l), i = rel % layer_in(l);
+  const uint16_t b = f2bf(x);
+  wk[w_off(l) + tc::kmaj_off(o, i, layer_in(l)) / 2] = b;
+  if (l > 0) wt[w_off(l) + tc::kmaj_off(i, o, layer_out(l)) / 2] = b;
+}
+__global__ void cast_kernel(const float* __restrict__ p, uint16_t* wk, uint16_t* wt) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < NPARAM) put_weight(q, p[q], wk, wt);
 }
 
-// Column sums of D [n][F] (BF16) over rows: per-CTA partials, then in order.
-__global__ void colsum_kernel(const uint16_t* __restrict__ D, int n, int F, int rows_per_cta, float* part) {
-  const int c = threadIdx.x;
-  if (c >= F) return;
-  const int r0 = blockIdx.x * rows_per_cta, r1 = min(n, r0 + rows_per_cta);
-  float t = 0.0f;
-  for (int r = r0; r < r1; ++r) t += bf2f(D[size_t(r) * F + c]);
-  part[size_t(blockIdx.x) * F + c] = t;
-}
-__global__ void colsum_reduce_kernel(const float* part, int nslot, int F, float* g, int boff, int used) {
-  const int c = threadIdx.x;
-  if (c >= F) return;
-  float t = 0.0f;
-  for (int k = 0; k < nslot; ++k) t += part[size_t(k) * F + c];
-  g[boff + c] = c < used ? t : 0.0f;
-}
-
-// dY = bf16(2 (y - t) / n) on the used outputs (0 elsewhere) and per-CTA
-// loss partials sum (y - t)^2.
-__global__ void loss_kernel(const float* __restrict__ Y, const float* __restrict__ T, int n, float inv_n,
-                            uint16_t* __restrict__ dY, double* lpart) {
-  __shared__ double red[8];
-  double s = 0.0;
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-    for (int q = 0; q < DO; ++q) {
-      float d = 0.0f;
-      if (q < DO_USED) {
-        const float e = Y[size_t(r) * DO + q] - T[size_t(r) * DO_USED + q];
-        s += double(e) * double(e);
-        d = 2.0f * e * inv_n;
-      }
-      dY[size_t(r) * DO + q] = f2bf(d);
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < int(blockDim.x / 32); ++w) t += red[w];
-    lpart[blockIdx.x] = t;
-  }
-}
-
-// Rows idx[k] (or k when idx is null) of X [*][16] -> BF16 [n][16]; of T
-// [*][4] -> [n][4].
-__global__ void gather_kernel(const float* __restrict__ X, const float* __restrict__ T, const int* __restrict__ idx,
-                              int n, uint16_t* __restrict__ Xb, float* __restrict__ Tb) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * DF; q += gridDim.x * blockDim.x) {
-    const int r = q / DF, f = q % DF;
-    const int s = idx ? idx[r] : r;
-    Xb[q] = f2bf(X[size_t(s) * DF + f]);
-    if (T && f < DO_USED) Tb[size_t(r) * DO_USED + f] = T[size_t(s) * DO_USED + f];
-  }
-}
-
-// Y [n][16] -> the used outputs [n][4].
-__global__ void take_outputs_kernel(const float* __restrict__ Y, int n, float* __restrict__ out) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n * DO_USED; q += gridDim.x * blockDim.x)
-    out[q] = Y[size_t(q / DO_USED) * DO + q % DO_USED];
-}
-
-// BF16 copies of the weights, row-major [out][in], and their transposes [in][out].
-__global__ void cast_kernel(const float* __restrict__ p, uint16_t* wb, uint16_t* wt) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < NPARAM; q += gridDim.x * blockDim.x) {
-    int l = 0;
-    while (l < NLAYER - 1 && q >= w_off(l + 1)) ++l;
-    const int rel = q - w_off(l), nw = layer_out(l) * layer_in(l);
-    if (rel >= nw) continue;  // a bias
-    const int o = rel / layer_in(l), i = rel % layer_in(l);
-    const uint16_t b = f2bf(p[q]);
-    wb[q] = b;
-    wt[w_off(l) + i * layer_out(l) + o] = b;
-  }
-}
-
-// Adam (Kingma & Ba, 2015).
-__global__ void adam_kernel(float* p, const float* g, float* m, float* v, int n, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
-  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
+// Adam (Kingma & Ba, 2015), the BF16 copies of the new weights, and the
+// step's loss from the clusters' sums.
+__global__ void adam_kernel(float* p, const float* __restrict__ g, float* m, float* v, float lr, float b1, float b2,
+                            float eps, float c1, float c2, uint16_t* wk, uint16_t* wt, const double* lpart, int nl,
+                            double rows, float* loss) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q < NPARAM) {
     const float gq = g[q];
     const float mq = b1 * m[q] + (1.0f - b1) * gq;
     const float vq = b2 * v[q] + (1.0f - b2) * gq * gq;
     m[q] = mq;
     v[q] = vq;
-    p[q] -= lr * (mq / c1) / (sqrtf(vq / c2) + eps);
+    const float x = p[q] - lr * (mq / c1) / (sqrtf(vq / c2) + eps);
+    p[q] = x;
+    put_weight(q, x, wk, wt);
+  }
+  if (q == 0 && loss) {
+    double t = 0.0;
+    for (int c = 0; c < nl; ++c) t += lpart[c];
+    *loss = float(t / rows);
   }
 }
 
@@ -368,158 +610,132 @@ struct Pcg {
   double uniform() { return (next() + 0.5) / 4294967296.0; }
 };
 
+constexpr int IDX_RING = 4;  // minibatch row lists on their way to the device
+
 }  // namespace
 
-// The network and its work arrays (rows: the capacity of one pass).
+// The network and its work arrays (cap: the rows of one pass).
 struct e2d_mlp_deep {
-  int device = 0, sms = 148, cap = 0, adam_t = 0;
+  int device = 0, sms = 148, cap = 0, icap = 0, hcap = 0, adam_t = 0;
   float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
-  uint16_t *wb = nullptr, *wt = nullptr;       // BF16 weights and transposes (param offsets)
-  uint16_t* xb = nullptr;                      // [cap][16]
-  uint16_t* act[DNL] = {};                     // H_1..H_4 [cap][256]
-  float* z[DNL] = {};                          // Z_1..Z_4 [cap][256]
-  float* y = nullptr;                          // [cap][16]
-  float* tb = nullptr;                         // [cap][4]
-  uint16_t* dy = nullptr;                      // [cap][16]
-  uint16_t* dz[2] = {};                        // [cap][256] ping-pong deltas
-  float* slots = nullptr;                      // [sms][256][256]
-  float* bpart = nullptr;                      // [sms][256]
-  double* lpart = nullptr;                     // [sms]
-  int* idx = nullptr;                          // [cap] minibatch rows
+  uint16_t *wk = nullptr, *wt = nullptr;       // BF16 weights and transposes (canonical tiles, param offsets)
+  uint16_t* xb = nullptr;                      // [cap][16] tiles
+  uint16_t* act[DNL] = {};                     // H_1..H_4, [cap][256] tiles
+  uint16_t* dy = nullptr;                      // [cap][16] tiles
+  uint16_t* dz[DNL] = {};                      // deltas of the hidden layers, [cap][256] tiles
+  float* gp = nullptr;                         // [CTAs][4][128 x 128] GELU' of the tiles in work
+  double* lpart = nullptr;                     // [clusters] loss sums
+  int* idx[IDX_RING] = {};                     // [icap] minibatch rows
+  int* hidx[IDX_RING] = {};                    // their pinned host copies
+  cudaEvent_t sent[IDX_RING] = {};             // the copy out of hidx is done
+  float* loss = nullptr;                       // [hcap] loss history of a training call
   int* err = nullptr;
-  std::vector<void*> ws;                       // work arrays (rebuilt on growth)
+  void* ws = nullptr;                          // the work arrays' memory (rebuilt on growth)
 };
 
 namespace {
 
-template <class T> bool dalloc(std::vector<void*>& v, T** p, size_t n) {
-  void* q = nullptr;
-  if (cudaMalloc(&q, sizeof(T) * (n ? n : 1)) != cudaSuccess) return false;
-  v.push_back(q);
-  *p = static_cast<T*>(q);
-  return true;
-}
-
 void free_ws(e2d_mlp_deep* d) {
-  for (void* q : d->ws) cudaFree(q);
-  d->ws.clear();
+  if (d->ws) cudaFree(d->ws);
+  d->ws = nullptr;
   d->cap = 0;
 }
 
+// CTAs of net_kernel over n rows: a pair per tile, at most one per SM.
+int net_grid(const e2d_mlp_deep* d, int n) {
+  const int ntiles = (n + TILE - 1) / TILE, most = d->sms / 2;
+  return 2 * (ntiles < most ? ntiles : most);
+}
+
+// Work arrays of a gradient over `rows` rows (whole tiles), one allocation.
 int ensure_cap(e2d_mlp_deep* d, int rows) {
   if (rows <= d->cap) return 0;
   free_ws(d);
-  const size_t c = size_t(rows);
-  bool ok = dalloc(d->ws, &d->xb, c * DF) && dalloc(d->ws, &d->y, c * DO) && dalloc(d->ws, &d->tb, c * DO_USED) &&
-            dalloc(d->ws, &d->dy, c * DO) && dalloc(d->ws, &d->dz[0], c * DH) && dalloc(d->ws, &d->dz[1], c * DH) &&
-            dalloc(d->ws, &d->idx, c);
-  for (int l = 0; l < DNL && ok; ++l) ok = dalloc(d->ws, &d->act[l], c * DH) && dalloc(d->ws, &d->z[l], c * DH);
-  if (!ok) {
-    free_ws(d);
+  const size_t c = (size_t(rows) + TILE - 1) / TILE * TILE, narrow = c * DF * 2, wide = c * DH * 2;
+  const size_t gp = size_t(net_grid(d, rows)) * DNL * TILE * HALF * 4;
+  if (cudaMalloc(&d->ws, 2 * narrow + 2 * DNL * wide + gp) != cudaSuccess) {
+    cudaGetLastError();
+    d->ws = nullptr;
     return E2D_ERR_NOMEM;
+  }
+  uint8_t* q = static_cast<uint8_t*>(d->ws);
+  auto take = [&](size_t bytes) { uint8_t* p = q; q += bytes; return p; };
+  d->gp = reinterpret_cast<float*>(take(gp));
+  d->xb = reinterpret_cast<uint16_t*>(take(narrow));
+  d->dy = reinterpret_cast<uint16_t*>(take(narrow));
+  for (int l = 0; l < DNL; ++l) {
+    d->act[l] = reinterpret_cast<uint16_t*>(take(wide));
+    d->dz[l] = reinterpret_cast<uint16_t*>(take(wide));
   }
   d->cap = rows;
   return 0;
 }
 
-size_t dense_smem(int K, int N) { return size_t(N) * K * 2 + size_t(TILE) * K * 2; }
-// The weight-gradient product holds up to 512 TMEM columns: a request above
-// half the SM's shared memory keeps it to one CTA per SM, so no CTA waits in
-// tcgen05.alloc for another's columns.
-size_t dw_smem(int N2) {
-  const size_t need = size_t(DH) * RC * 2 + size_t(N2) * RC * 2;
-  return need < 120 * 1024 ? 120 * 1024 : need;
-}
-
-template <int EPI>
-int dense(e2d_mlp_deep* d, const uint16_t* A, int K, const uint16_t* Bw, int N, const float* bias, int n, float* Z,
-          uint16_t* H, const float* Zp, float* Y, cudaStream_t st) {
-  const size_t smem = dense_smem(K, N);
-  if (cudaFuncSetAttribute(dense_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return E2D_ERR_CUDA;
-  const int ntiles = (n + TILE - 1) / TILE;
-  dense_kernel<EPI><<<ntiles < d->sms ? ntiles : d->sms, TILE, smem, st>>>(A, K, Bw, N, bias, n, Z, H, Zp, Y,
-                                                                           d->err);
-  return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
-}
-
-// Forward pass over n rows already in d->xb: activations, pre-activations
-// and the outputs d->y.
-int forward_rows(e2d_mlp_deep* d, int n, cudaStream_t st) {
-  int rc;
-  const uint16_t* a = d->xb;
-  for (int l = 0; l < DNL; ++l) {
-    if ((rc = dense<FWD_GELU>(d, a, layer_in(l), d->wb + w_off(l), DH, d->p + b_off(l), n, d->z[l], d->act[l],
-                              nullptr, nullptr, st)))
-      return rc;
-    a = d->act[l];
+void free_train(e2d_mlp_deep* d) {
+  for (int k = 0; k < IDX_RING; ++k) {
+    if (d->idx[k]) cudaFree(d->idx[k]);
+    if (d->hidx[k]) cudaFreeHost(d->hidx[k]);
+    if (d->sent[k]) cudaEventDestroy(d->sent[k]);
+    d->idx[k] = d->hidx[k] = nullptr;
+    d->sent[k] = nullptr;
   }
-  return dense<FWD_LINEAR>(d, a, DH, d->wb + w_off(DNL), DO, d->p + b_off(DNL), n, nullptr, nullptr, nullptr, d->y,
-                           st);
+  if (d->loss) cudaFree(d->loss);
+  d->loss = nullptr;
+  d->icap = d->hcap = 0;
 }
 
-int weight_grad(e2d_mlp_deep* d, const uint16_t* P, const uint16_t* Q, int N2, int n, int woff, int transpose,
-                cudaStream_t st) {
-  const size_t smem = dw_smem(N2);
-  if (cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)
-    return E2D_ERR_CUDA;
-  int rows = (n + d->sms - 1) / d->sms;
-  rows = ((rows + RC - 1) / RC) * RC;
-  const int grid = (n + rows - 1) / rows;
-  dw_kernel<<<grid, TILE, smem, st>>>(P, Q, N2, n, rows, d->slots, d->err);
-  dw_reduce_kernel<<<64, 256, 0, st>>>(d->slots, grid, N2, d->g, woff, transpose);
-  return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
-}
-
-int bias_grad(e2d_mlp_deep* d, const uint16_t* D, int F, int n, int boff, int used, cudaStream_t st) {
-  const int rows = (n + d->sms - 1) / d->sms;
-  const int grid = (n + rows - 1) / rows;
-  colsum_kernel<<<grid, 256, 0, st>>>(D, n, F, rows, d->bpart);
-  colsum_reduce_kernel<<<1, 256, 0, st>>>(d->bpart, grid, F, d->g, boff, used);
-  return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
-}
-
-// Gradient of loss = sum over rows and the used outputs of (y - t)^2 / n
-// for the n rows in d->xb / d->tb, into d->g; the loss sum into *lsum.
-int gradient_rows(e2d_mlp_deep* d, int n, double* lsum, cudaStream_t st) {
-  int rc;
-  if ((rc = forward_rows(d, n, st))) return rc;
-  const int lgrid = d->sms;
-  loss_kernel<<<lgrid, 256, 0, st>>>(d->y, d->tb, n, 1.0f / float(n), d->dy, d->lpart);
-  if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
-  // output layer: dW5^T = H4^T dY (transposed into W5), db5 = column sums of dY
-  if ((rc = weight_grad(d, d->act[DNL - 1], d->dy, DO, n, w_off(DNL), 1, st)) ||
-      (rc = bias_grad(d, d->dy, DO, n, b_off(DNL), DO_USED, st)))
-    return rc;
-  // dZ4 = (dY W5) * gelu'(Z4): A = dY [n][16], B = W5^T [256][16]
-  if ((rc = dense<BWD_GELU>(d, d->dy, DO, d->wt + w_off(DNL), DH, nullptr, n, nullptr, d->dz[0], d->z[DNL - 1],
-                            nullptr, st)))
-    return rc;
-  int cur = 0;
-  for (int l = DNL - 1; l >= 0; --l) {
-    const uint16_t* dz = d->dz[cur];
-    const uint16_t* ain = l == 0 ? d->xb : d->act[l - 1];
-    // dW_l = dZ^T A_in [256][in], db_l = column sums of dZ
-    if ((rc = weight_grad(d, dz, ain, layer_in(l), n, w_off(l), 0, st)) ||
-        (rc = bias_grad(d, dz, DH, n, b_off(l), DH, st)))
-      return rc;
-    if (l == 0) break;
-    // dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): B = W_l^T [256 in][256 out]
-    if ((rc = dense<BWD_GELU>(d, dz, DH, d->wt + w_off(l), DH, nullptr, n, nullptr, d->dz[cur ^ 1], d->z[l - 1],
-                              nullptr, st)))
-      return rc;
-    cur ^= 1;
+// The row lists of minibatches of `batch` rows and a history of `steps` losses.
+int ensure_train(e2d_mlp_deep* d, int batch, int steps) {
+  if (batch <= d->icap && steps <= d->hcap) return 0;
+  if (batch < d->icap) batch = d->icap;
+  if (steps < d->hcap) steps = d->hcap;
+  free_train(d);
+  bool ok = cudaMalloc(&d->loss, sizeof(float) * size_t(steps > 0 ? steps : 1)) == cudaSuccess;
+  for (int k = 0; k < IDX_RING && ok; ++k)
+    ok = cudaMalloc(&d->idx[k], sizeof(int) * size_t(batch)) == cudaSuccess &&
+         cudaMallocHost(&d->hidx[k], sizeof(int) * size_t(batch)) == cudaSuccess &&
+         cudaEventCreateWithFlags(&d->sent[k], cudaEventDisableTiming) == cudaSuccess;
+  if (!ok) {
+    free_train(d);
+    return E2D_ERR_NOMEM;
   }
-  if (lsum) {
-    std::vector<double> lp(lgrid);
-    if (cudaMemcpyAsync(lp.data(), d->lpart, sizeof(double) * lgrid, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      return E2D_ERR_CUDA;
-    double t = 0.0;
-    for (double x : lp) t += x;
-    *lsum = t;
-  }
+  d->icap = batch;
+  d->hcap = steps;
   return 0;
+}
+
+NetArgs net_args(const e2d_mlp_deep* d, const float* X, const float* T, const int* idx, int n, float* Y) {
+  NetArgs a{};
+  a.X = X; a.T = T; a.idx = idx; a.Y = Y;
+  a.vec = ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(T) | reinterpret_cast<uintptr_t>(Y)) & 15) == 0;
+  a.n = n;
+  a.inv_n = 1.0f / float(n);
+  a.wk = d->wk; a.wt = d->wt; a.p = d->p;
+  a.xb = d->xb; a.dy = d->dy;
+  for (int l = 0; l < DNL; ++l) { a.act[l] = d->act[l]; a.dz[l] = d->dz[l]; }
+  a.gp = d->gp;
+  a.lpart = d->lpart;
+  a.err = d->err;
+  return a;
+}
+
+// Gradient of loss = sum over rows and the used outputs of (y - t)^2 / n over
+// n rows (idx, or the first n) into d->g; the loss sums into d->lpart.  The
+// rows are grouped as one group per SM, so that the sums' order depends on n
+// alone.
+int gradient_rows(e2d_mlp_deep* d, const float* X, const float* T, const int* idx, int n, cudaStream_t st) {
+  net_kernel<true><<<net_grid(d, n), NT, sizeof(NetSmem), st>>>(net_args(d, X, T, idx, n, nullptr));
+  if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
+  DwArgs w{};
+  w.xb = d->xb; w.dy = d->dy;
+  for (int l = 0; l < DNL; ++l) { w.act[l] = d->act[l]; w.dz[l] = d->dz[l]; }
+  w.n = n;
+  w.brows = (n + d->sms - 1) / d->sms;
+  w.rows = (w.brows + RC - 1) / RC * RC;
+  w.g = d->g;
+  w.err = d->err;
+  dw_kernel<<<DW_ITEMS + DW_BIAS, DW_THREADS, sizeof(DwSmem), st>>>(w);
+  return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
 }
 
 int check_err(e2d_mlp_deep* d, cudaStream_t st) {
@@ -531,7 +747,7 @@ int check_err(e2d_mlp_deep* d, cudaStream_t st) {
 }
 
 int refresh(e2d_mlp_deep* d, cudaStream_t st) {
-  cast_kernel<<<256, 256, 0, st>>>(d->p, d->wb, d->wt);
+  cast_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(d->p, d->wk, d->wt);
   return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
 }
 
@@ -547,11 +763,16 @@ e2d_mlp_deep* e2d_mlp_deep_create(uint64_t seed, int* err) {
   std::vector<void*> fixed;
   bool ok = cudaMalloc(&d->p, 4 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->g, 4 * size_t(NPARAM)) == cudaSuccess &&
             cudaMalloc(&d->m, 4 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->v, 4 * size_t(NPARAM)) == cudaSuccess &&
-            cudaMalloc(&d->wb, 2 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->wt, 2 * size_t(NPARAM)) == cudaSuccess &&
-            cudaMalloc(&d->slots, 4 * size_t(d->sms) * DH * DH) == cudaSuccess &&
-            cudaMalloc(&d->bpart, 4 * size_t(d->sms) * DH) == cudaSuccess &&
+            cudaMalloc(&d->wk, 2 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->wt, 2 * size_t(NPARAM)) == cudaSuccess &&
             cudaMalloc(&d->lpart, sizeof(double) * d->sms) == cudaSuccess &&
             cudaMalloc(&d->err, sizeof(int)) == cudaSuccess;
+  if (ok && (cudaFuncSetAttribute(net_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(NetSmem))) ||
+             cudaFuncSetAttribute(net_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(NetSmem))) ||
+             cudaFuncSetAttribute(dw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(DwSmem))))) {
+    if (err) *err = E2D_ERR_CUDA;
+    e2d_mlp_deep_destroy(d);
+    return nullptr;
+  }
   if (!ok) {
     if (err) *err = E2D_ERR_NOMEM;
     e2d_mlp_deep_destroy(d);
@@ -573,7 +794,8 @@ e2d_mlp_deep* e2d_mlp_deep_create(uint64_t seed, int* err) {
   }
   if (cudaMemcpy(d->p, h.data(), 4 * size_t(NPARAM), cudaMemcpyHostToDevice) != cudaSuccess ||
       cudaMemset(d->m, 0, 4 * size_t(NPARAM)) != cudaSuccess || cudaMemset(d->v, 0, 4 * size_t(NPARAM)) != cudaSuccess ||
-      cudaMemset(d->g, 0, 4 * size_t(NPARAM)) != cudaSuccess || cudaMemset(d->wt, 0, 2 * size_t(NPARAM)) != cudaSuccess ||
+      cudaMemset(d->g, 0, 4 * size_t(NPARAM)) != cudaSuccess || cudaMemset(d->wk, 0, 2 * size_t(NPARAM)) != cudaSuccess ||
+      cudaMemset(d->wt, 0, 2 * size_t(NPARAM)) != cudaSuccess ||
       cudaMemset(d->err, 0, sizeof(int)) != cudaSuccess || refresh(d, 0) || cudaDeviceSynchronize() != cudaSuccess) {
     if (err) *err = E2D_ERR_CUDA;
     e2d_mlp_deep_destroy(d);
@@ -585,8 +807,9 @@ e2d_mlp_deep* e2d_mlp_deep_create(uint64_t seed, int* err) {
 void e2d_mlp_deep_destroy(e2d_mlp_deep* d) {
   if (!d) return;
   free_ws(d);
-  for (void* q : {(void*)d->p, (void*)d->g, (void*)d->m, (void*)d->v, (void*)d->wb, (void*)d->wt, (void*)d->slots,
-                  (void*)d->bpart, (void*)d->lpart, (void*)d->err})
+  free_train(d);
+  for (void* q : {(void*)d->p, (void*)d->g, (void*)d->m, (void*)d->v, (void*)d->wk, (void*)d->wt, (void*)d->lpart,
+                  (void*)d->err})
     if (q) cudaFree(q);
   delete d;
 }
@@ -606,17 +829,8 @@ int e2d_mlp_deep_params(e2d_mlp_deep* d, float* out, const float* in) {
 int e2d_mlp_deep_forward(e2d_mlp_deep* d, const float* X, int n, float* Y, void* stream) {
   if (!d || !X || !Y || n < 1) return E2D_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int chunk = n < 65536 ? n : 65536;
-  int rc;
-  if ((rc = ensure_cap(d, chunk))) return rc;
-  for (int r0 = 0; r0 < n; r0 += chunk) {
-    const int m = n - r0 < chunk ? n - r0 : chunk;
-    gather_kernel<<<256, 256, 0, st>>>(X + size_t(r0) * DF, nullptr, nullptr, m, d->xb, nullptr);
-    if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
-    if ((rc = forward_rows(d, m, st))) return rc;
-    take_outputs_kernel<<<256, 256, 0, st>>>(d->y, m, Y + size_t(r0) * DO_USED);
-    if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
-  }
+  net_kernel<false><<<net_grid(d, n), NT, sizeof(NetSmem), st>>>(net_args(d, X, nullptr, nullptr, n, Y));
+  if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
   return check_err(d, st);
 }
 
@@ -625,48 +839,63 @@ int e2d_mlp_deep_gradient(e2d_mlp_deep* d, const float* X, const float* T, int n
   if (!d || !X || !T || n < 1) return E2D_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   int rc;
-  if ((rc = ensure_cap(d, n))) return rc;
-  gather_kernel<<<256, 256, 0, st>>>(X, T, nullptr, n, d->xb, d->tb);
-  if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
-  double l = 0.0;
-  if ((rc = gradient_rows(d, n, &l, st)) || (rc = check_err(d, st))) return rc;
+  if ((rc = ensure_cap(d, n)) || (rc = gradient_rows(d, X, T, nullptr, n, st))) return rc;
+  const int nl = net_grid(d, n) / 2;
+  std::vector<double> lp(nl);
+  if (cudaMemcpyAsync(lp.data(), d->lpart, sizeof(double) * nl, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    return E2D_ERR_CUDA;
+  if ((rc = check_err(d, st))) return rc;
   if (grad && cudaMemcpy(grad, d->g, 4 * size_t(NPARAM), cudaMemcpyDeviceToHost) != cudaSuccess) return E2D_ERR_CUDA;
+  double l = 0.0;
+  for (double x : lp) l += x;
   if (loss) *loss = l / double(n);
   return 0;
 }
 
+// Three launches a step and no wait for the device: the host draws the next
+// minibatches' rows (through a ring of pinned lists) while the device works,
+// and reads the losses once at the end.
 int e2d_mlp_deep_train(e2d_mlp_deep* d, const float* X, const float* T, int n, int steps, int batch, float lr,
                        uint64_t seed, float* loss_hist, void* stream) {
   if (!d || !X || !T || n < 1 || steps < 0 || batch < 1 || !(lr > 0.0f)) return E2D_ERR_ARG;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int b = batch < n ? batch : n;
   int rc;
-  if ((rc = ensure_cap(d, b))) return rc;
+  if ((rc = ensure_cap(d, b)) || (rc = ensure_train(d, b, steps))) return rc;
   Pcg rng{seed * 2 + 1, (seed << 1) | 1};
-  std::vector<int> perm(n), hidx(b);
+  std::vector<int> perm(n);
   for (int q = 0; q < n; ++q) perm[q] = q;
   int pos = n;  // reshuffle at the first step
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const int nl = net_grid(d, b) / 2;
   for (int k = 0; k < steps; ++k) {
-    for (int q = 0; q < b; ++q) {
+    const int slot = k % IDX_RING;
+    // the list's last copy to the device is done (an earlier call's included)
+    if (cudaEventSynchronize(d->sent[slot]) != cudaSuccess) return E2D_ERR_CUDA;
+    int* hidx = d->hidx[slot];
+    for (int q = 0; q < b;) {
       if (pos >= n) {  // Fisher-Yates shuffle of the rows per epoch
         for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[int(rng.next() % uint32_t(i + 1))]);
         pos = 0;
       }
-      hidx[q] = perm[pos++];
+      const int take = b - q < n - pos ? b - q : n - pos;
+      std::copy(perm.begin() + pos, perm.begin() + pos + take, hidx + q);
+      q += take;
+      pos += take;
     }
-    if (cudaMemcpyAsync(d->idx, hidx.data(), sizeof(int) * b, cudaMemcpyHostToDevice, st) != cudaSuccess)
+    if (cudaMemcpyAsync(d->idx[slot], hidx, sizeof(int) * b, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+        cudaEventRecord(d->sent[slot], st) != cudaSuccess)
       return E2D_ERR_CUDA;
-    gather_kernel<<<256, 256, 0, st>>>(X, T, d->idx, b, d->xb, d->tb);
-    if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
-    double l = 0.0;
-    if ((rc = gradient_rows(d, b, loss_hist ? &l : nullptr, st))) return rc;
-    if (loss_hist) loss_hist[k] = float(l / double(b));
+    if ((rc = gradient_rows(d, X, T, d->idx[slot], b, st))) return rc;
     ++d->adam_t;
     const float c1 = 1.0f - powf(b1, float(d->adam_t)), c2 = 1.0f - powf(b2, float(d->adam_t));
-    adam_kernel<<<256, 256, 0, st>>>(d->p, d->g, d->m, d->v, NPARAM, lr, b1, b2, eps, c1, c2);
-    if (cudaGetLastError() != cudaSuccess || refresh(d, st)) return E2D_ERR_CUDA;
+    adam_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(d->p, d->g, d->m, d->v, lr, b1, b2, eps, c1, c2, d->wk, d->wt,
+                                                      d->lpart, nl, double(b), loss_hist ? d->loss + k : nullptr);
+    if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
   }
+  if (loss_hist && steps > 0 &&
+      cudaMemcpyAsync(loss_hist, d->loss, sizeof(float) * size_t(steps), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+    return E2D_ERR_CUDA;
   return check_err(d, st);
 }
 
