@@ -32,6 +32,7 @@
 
 #include "e2d_geom.cuh"
 #include "e2d_handle.h"
+#include "e2d_tc.cuh"
 
 using namespace e2d;
 
@@ -591,9 +592,10 @@ struct GmresDev {
   int m, ncase;                    // m: the buffers' cycle length (array strides)
   const int* cfg;                  // device: [0] cycle length of this solve (<= m), [1] iteration cap
   double *H, *cs, *sn, *sv;        // [C][m][m+1], [C][m], [C][m], [C][m+1]
+  double* run;                     // [C][m+1] right-hand side entry a step's rotation takes up
   double *resid0, *relres, *tol;   // [C]
   int *iters, *flags, *jstop;      // [C]
-  int* its;                        // iterations of this GMRES solve (all cases in lockstep)
+  int* its;                        // iterations of this GMRES solve before the current cycle (all cases in lockstep)
   int* err;                        // first error (E2D_ERR_*), 0 = none
   int* progress;                   // host-mapped [m]: cases still iterating after step j
 };
@@ -613,6 +615,7 @@ __global__ void gmres_cycle_start_kernel(GmresDev G, const double* nrm, int* act
     double* sv = G.sv + size_t(c) * (G.m + 1);
     sv[0] = beta;
     for (int q = 1; q <= G.cfg[0]; ++q) sv[q] = 0.0;
+    G.run[size_t(c) * (G.m + 1)] = beta;
     if (first) G.resid0[c] = beta;
     G.flags[c] = 0;
     G.jstop[c] = -1;
@@ -631,6 +634,21 @@ __device__ __forceinline__ void apply_rot(double& dx, double& dy, double cs, dou
   dx = t;
 }
 
+// generate_rotation (GMRES2D.h:761-775).
+__device__ __forceinline__ void make_rot(double dx, double dy, double& cj, double& sj) {
+  if (dy == 0.0) {
+    cj = 1.0; sj = 0.0;
+  } else if (fabs(dy) > fabs(dx)) {
+    const double t = dx / dy;
+    sj = 1.0 / sqrt(1.0 + t * t);
+    cj = t * sj;
+  } else {
+    const double t = dy / dx;
+    cj = 1.0 / sqrt(1.0 + t * t);
+    sj = t * cj;
+  }
+}
+
 // End of Arnoldi step j: per iterating case, the Hessenberg column (hcol,
 // [j+2][ncase]) takes the previous rotations, a new rotation zeroes its
 // subdiagonal, the right-hand side rotates with it, and the stop test
@@ -638,7 +656,7 @@ __device__ __forceinline__ void apply_rot(double& dx, double& dy, double cs, dou
 __global__ void gmres_givens_kernel(GmresDev G, const double* hcol, int* active, int j) {
   __shared__ int its, count;
   if (threadIdx.x == 0) {
-    its = ++*G.its;
+    its = *G.its + j + 1;
     count = 0;
   }
   __syncthreads();
@@ -664,20 +682,8 @@ __global__ void gmres_givens_kernel(GmresDev G, const double* hcol, int* active,
     if (!isfinite(hlast)) gm_error(G, E2D_ERR_NAN);
     Hj[j] = a;
     Hj[j + 1] = hlast;
-    // generate_rotation (GMRES2D.h:761-775)
-    const double dx = Hj[j], dy = Hj[j + 1];
     double cj, sj;
-    if (dy == 0.0) {
-      cj = 1.0; sj = 0.0;
-    } else if (fabs(dy) > fabs(dx)) {
-      const double t = dx / dy;
-      sj = 1.0 / sqrt(1.0 + t * t);
-      cj = t * sj;
-    } else {
-      const double t = dy / dx;
-      cj = 1.0 / sqrt(1.0 + t * t);
-      sj = t * cj;
-    }
+    make_rot(Hj[j], Hj[j + 1], cj, sj);
     cs[j] = cj; sn[j] = sj;
     apply_rot(Hj[j], Hj[j + 1], cj, sj);
     apply_rot(sv[j], sv[j + 1], cj, sj);
@@ -708,6 +714,7 @@ __global__ void gmres_givens_kernel(GmresDev G, const double* hcol, int* active,
 // x update, and the cases that met the tolerance or the cap are done.
 __global__ void gmres_backsub_kernel(GmresDev G, double* svals, int* kcount) {
   const int m = G.m;
+  if (threadIdx.x == 0) *G.its += G.cfg[0];  // a case that goes on took the whole cycle
   for (int c = threadIdx.x; c < G.ncase; c += blockDim.x) {
     kcount[c] = 0;
     const int f = G.flags[c];
@@ -725,6 +732,8 @@ __global__ void gmres_backsub_kernel(GmresDev G, double* svals, int* kcount) {
     if (f & (GF_MET | GF_FAILED)) G.flags[c] = f | GF_DONE;
   }
 }
+
+#include "e2d_arnoldi.cuh"
 
 }  // namespace
 
@@ -747,6 +756,13 @@ struct e2d_nks_state {
   double* Z = nullptr;       // m * n
   double* partial = nullptr; // [nblk * ch]
   unsigned* counter = nullptr; // [ncase] arrivals of the reduction CTAs
+  int team = 0;              // arnoldi_kernel: 1 a cluster per case, 2 a share of the GPU per case, 0 separate kernels
+  int team_ctas = 0, team_ctaslots = 0, team_slots = 0;
+  size_t team_smem = 0;
+  int* team_cnt = nullptr;   // [2]
+  int* team_cta0 = nullptr;                   // [ncase + 1]
+  ulonglong2* team_part = nullptr;
+  unsigned long long* team_round = nullptr;   // [ncase]
   int ch_vec = 1, ch_cell = 1; // CTAs per block of the vector / per-cell reductions
   std::vector<cudaGraphExec_t> graphs;  // Arnoldi step j, captured on its second use
   std::vector<int> graph_uses;
@@ -823,6 +839,118 @@ template <class T> int nalloc(e2d_nks_state* s, T** p, size_t n) {
   return 0;
 }
 
+// Bytes of the work area of arnoldi_kernel's CTAs for a case of nb blocks on a
+// team of `size` CTAs: the most vector entries or cells one of them holds.
+size_t team_work(const e2d_handle* h, int nb, int size) {
+  const e2d_nks_state* s = h->nks;
+  const int cpb = h->B.NCi * h->B.NCj, nper2 = s->nper4 / 2;
+  const int len = (nper2 + s->ch_vec - 1) / s->ch_vec, lenc = (cpb + s->ch_cell - 1) / s->ch_cell;
+  const long long ns = (long long)nb * s->ch_vec, nsc = (long long)nb * s->ch_cell;
+  return std::max(size_t((ns + size - 1) / size) * len, size_t((nsc + size - 1) / size) * lenc * 2) * sizeof(double2);
+}
+
+// How the Arnoldi steps of this handle run: a cluster of 16 CTAs per case
+// where every case's vector fits the clusters' registers (64 slots of 512
+// entries, 12 blocks of 32 x 32; a quarter more in shared memory still wins)
+// and all clusters run at once; else a share of a cooperative launch per
+// case, by the cases' sizes, up to 8 slots a CTA (past that the vectors'
+// traffic through one SM costs more than the launches it saves) and a case
+// for every four SMs; else the separate kernels.  Measured on B200, ms for 4
+// Newton steps, block Jacobi, separate kernels / cluster / share of the GPU:
+// 4 blocks of 32 x 32 22.1 / 12.6 / 17.0, 12 blocks 34.7 / 19.6 / 28.5, 16 blocks 58.4
+// / 43.4 / 48.4, 24 blocks 61.9 / 58.6 / 51.8, 48 blocks 46.7 / 80.6 / 32.4, 96
+// blocks 70.1 / - / 50.5; batches, 3 steps: 3 cases of 8 to 16 blocks 26.7 /
+// 16.6 / 17.8, 6 of 8 to 24 41.3 / 35.5 / 28.8, 8 of 8 to 48 (7 slots a CTA) 56.7 /
+// 57.4 / 53.6, 11 of 8 to 96 (14 slots) 99 / - / 122.
+int team_setup(e2d_handle* h) {
+  e2d_nks_state* s = h->nks;
+  const Blocks& B = h->B;
+  const int C = s->ncase;
+  std::vector<int> start{0, B.nblk};
+  if (B.case_start) {
+    start.resize(C + 1);
+    E2D_CK(cudaMemcpyAsync(start.data(), B.case_start, sizeof(int) * (C + 1), cudaMemcpyDeviceToHost, h->stream));
+    E2D_CK(cudaStreamSynchronize(h->stream));
+  }
+  int optin = 0, sms = 0, coop = 0, rc;
+  E2D_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device));
+  E2D_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+  E2D_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->device));
+  const int maxch = std::max(s->ch_vec, s->ch_cell);
+  int nbmax = 0;
+  for (int c = 0; c < C; ++c) nbmax = std::max(nbmax, start[c + 1] - start[c]);
+  s->team = 0;
+  if ((rc = nalloc(s, &s->team_cnt, 2)) || (rc = nalloc(s, &s->team_round, C)) ||
+      (rc = nalloc(s, &s->team_cta0, C + 1)) ||
+      (rc = nalloc(s, &s->team_part, 2 * (size_t(B.nblk) * maxch + sms))))
+    return rc;
+  E2D_CK(cudaMemsetAsync(s->team_cnt, 0, 2 * sizeof(int), h->stream));
+  E2D_CK(cudaMemsetAsync(s->team_round, 0, sizeof(unsigned long long) * C, h->stream));
+  E2D_CK(cudaMemsetAsync(s->team_part, 0, sizeof(ulonglong2) * 2 * (size_t(B.nblk) * maxch + sms), h->stream));
+  // the Arnoldi kernel's shared memory with `slots` slots a CTA
+  auto smem = [&](int slots, int all, size_t work) { return arnoldi_head(slots, all, s->m) + work; };
+  auto slots_of = [&](int nb, int size) { return (nb * maxch + size - 1) / size; };
+  size_t work = 0;
+  for (int c = 0; c < C; ++c) work = std::max(work, team_work(h, start[c + 1] - start[c], ATEAM));
+  const int cluster_slots = slots_of(nbmax, ATEAM);
+  if (cluster_slots <= AREG * AGROUPS + 1 && smem(cluster_slots, 0, work) <= size_t(optin) &&
+      cudaFuncSetAttribute(arnoldi_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+      cudaFuncSetAttribute(arnoldi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess) {
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ATEAM; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(ATEAM * C); cfg.blockDim = dim3(AT); cfg.dynamicSmemBytes = smem(cluster_slots, 0, work);
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, arnoldi_kernel<true>, &cfg) == cudaSuccess && n >= C) {
+      s->team = 1;
+      s->team_ctas = ATEAM * C;
+      s->team_ctaslots = cluster_slots;
+      s->team_smem = cfg.dynamicSmemBytes;
+      return 0;
+    }
+  }
+  cudaGetLastError();
+  if (!coop || 4 * C > sms) return 0;
+  // CTAs by the cases' blocks, at least one each, the rest where a CTA holds most
+  std::vector<int> size(C), cta0(C + 1, 0);
+  int left = sms;
+  for (int c = 0; c < C; ++c) {
+    size[c] = std::max(1, int((long long)(sms - C) * (start[c + 1] - start[c]) / B.nblk));
+    left -= size[c];
+  }
+  for (; left > 0; --left) {
+    int m = 0;
+    for (int c = 1; c < C; ++c)
+      if ((long long)(start[c + 1] - start[c]) * size[m] > (long long)(start[m + 1] - start[m]) * size[c]) m = c;
+    ++size[m];
+  }
+  work = 0;
+  int slots = 0, all = 0;
+  for (int c = 0; c < C; ++c) {
+    cta0[c + 1] = cta0[c] + size[c];
+    work = std::max(work, team_work(h, start[c + 1] - start[c], size[c]));
+    slots = std::max(slots, slots_of(start[c + 1] - start[c], size[c]));
+    all = std::max(all, team_slots(start[c + 1] - start[c], maxch, size[c]));
+  }
+  int n = 0;
+  if (slots <= 8 && smem(slots, all, work) <= size_t(optin) &&
+      cudaFuncSetAttribute(arnoldi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin) == cudaSuccess &&
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, arnoldi_kernel<false>, AT, smem(slots, all, work)) == cudaSuccess &&
+      n > 0) {
+    E2D_CK(cudaMemcpyAsync(s->team_cta0, cta0.data(), sizeof(int) * (C + 1), cudaMemcpyHostToDevice, h->stream));
+    E2D_CK(cudaStreamSynchronize(h->stream));
+    s->team = 2;
+    s->team_ctas = sms;
+    s->team_ctaslots = slots;
+    s->team_slots = all;
+    s->team_smem = smem(slots, all, work);
+  }
+  cudaGetLastError();
+  return 0;
+}
+
 int nks_setup(e2d_handle* h, int m) {
   if (h->nks && h->nks->m >= m) return 0;
   nks_free(h);
@@ -855,6 +983,7 @@ int nks_setup(e2d_handle* h, int m) {
   G.ncase = C;
   if ((rc = nalloc(s, &G.H, size_t(C) * m * (m + 1))) || (rc = nalloc(s, &G.cs, size_t(C) * m)) ||
       (rc = nalloc(s, &G.sn, size_t(C) * m)) || (rc = nalloc(s, &G.sv, size_t(C) * (m + 1))) ||
+      (rc = nalloc(s, &G.run, size_t(C) * (m + 1))) ||
       (rc = nalloc(s, &G.resid0, C)) || (rc = nalloc(s, &G.relres, C)) || (rc = nalloc(s, &G.tol, C)) ||
       (rc = nalloc(s, &G.iters, C)) || (rc = nalloc(s, &G.flags, C)) || (rc = nalloc(s, &G.jstop, C)) ||
       (rc = nalloc(s, &G.its, 1)) || (rc = nalloc(s, &G.err, 1)) || (rc = nalloc(s, &s->gcfg, 2))) {
@@ -886,6 +1015,10 @@ int nks_setup(e2d_handle* h, int m) {
   s->ch_cell = std::max(1, std::min(16, h->B.NCi * h->B.NCj / 512));
   identity_blocks_kernel<<<VGRID, VT, 0, h->stream>>>(s->Minv, (long long)h->ncell);
   E2D_CK(cudaGetLastError());
+  if ((rc = team_setup(h))) {
+    nks_free(h);
+    return rc;
+  }
   return 0;
 }
 
@@ -1137,6 +1270,61 @@ int arnoldi_step(e2d_handle* h, int j, double eps0, const Norm4& nm, bool ilu) {
   return 0;
 }
 
+// arnoldi_kernel for step j (mgs: orthogonalise v_{j+1} and test for the end)
+// and what the next step starts with.
+int launch_arnoldi(e2d_handle* h, int j, bool mgs, int next, double eps0, const Norm4& nm) {
+  e2d_nks_state* s = h->nks;
+  ArnoldiArgs a{};
+  a.B = h->B;
+  a.G = s->gd;
+  a.V = s->V; a.Z = s->Z; a.Minv = s->Minv; a.Uo = s->Uo; a.eps = s->eps; a.active = s->active;
+  a.cnt = s->team_cnt; a.gpart = s->team_part; a.ground = s->team_round; a.cta0 = s->team_cta0;
+  a.n = s->n;
+  a.eps0 = eps0;
+  a.nm = nm;
+  a.j = j; a.mgs = mgs; a.next = next;
+  a.nper2 = s->nper4 / 2; a.ch = s->ch_vec; a.len = (a.nper2 + a.ch - 1) / a.ch;
+  a.cpb = h->B.NCi * h->B.NCj; a.chc = s->ch_cell; a.lenc = (a.cpb + a.chc - 1) / a.chc;
+  a.maxch = std::max(s->ch_vec, s->ch_cell);
+  a.ctaslots = s->team_ctaslots; a.teamslots = s->team_slots;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute at{};
+  if (s->team == 1) {
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ATEAM; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  } else {
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+  }
+  cfg.gridDim = dim3(s->team_ctas); cfg.blockDim = dim3(AT); cfg.dynamicSmemBytes = s->team_smem;
+  cfg.stream = h->stream; cfg.attrs = &at; cfg.numAttrs = 1;
+  E2D_CK(s->team == 1 ? cudaLaunchKernelEx(&cfg, arnoldi_kernel<true>, a) : cudaLaunchKernelEx(&cfg, arnoldi_kernel<false>, a));
+  return 0;
+}
+
+// The head of step j (its z_j = M^-1 v_j, eps and perturbed state) where it
+// does not follow a step in the same kernel: the start of a cycle, and every
+// step with ILU(k).
+int arnoldi_head_step(e2d_handle* h, int j, double eps0, const Norm4& nm, bool ilu) {
+  e2d_nks_state* s = h->nks;
+  int rc;
+  if (ilu && (rc = ilu_apply(h, s->V + size_t(j) * s->n, s->Z + size_t(j) * s->n))) return rc;
+  return launch_arnoldi(h, j - 1, false, ilu ? NEXT_PERTURB : NEXT_JACOBI, eps0, nm);
+}
+
+// Arnoldi step j with arnoldi_kernel: the Frechet product of the perturbed
+// state its head left, then one kernel to the next step's head.
+int arnoldi_team_step(e2d_handle* h, int j, double eps0, const Norm4& nm, bool ilu) {
+  e2d_nks_state* s = h->nks;
+  int rc;
+  E2D_CK(ghost_fill_for(h, 0));
+  E2D_CK(launch_frechet(h, s->Z + size_t(j) * s->n, s->V + size_t(j + 1) * s->n, nm));
+  const bool more = j + 1 < s->m;
+  if ((rc = launch_arnoldi(h, j, true, more && !ilu ? NEXT_JACOBI : NEXT_NONE, eps0, nm))) return rc;
+  if (ilu && more) return arnoldi_head_step(h, j + 1, eps0, nm, true);
+  return 0;
+}
+
 // Arnoldi step j through a CUDA graph: the first use of a j runs eagerly,
 // the second captures the step, later uses replay it (one launch instead of
 // about 2j + 8).  Every pointer the step reads is fixed for the life of the
@@ -1154,10 +1342,11 @@ int run_arnoldi(e2d_handle* h, int j, double eps0, const Norm4& nm, bool ilu) {
     E2D_CK(cudaGraphLaunch(s->graphs[j], h->stream));
     return 0;
   }
-  if (s->graph_uses[j]++ == 0) return arnoldi_step(h, j, eps0, nm, ilu);
+  auto step = [&]() { return s->team ? arnoldi_team_step(h, j, eps0, nm, ilu) : arnoldi_step(h, j, eps0, nm, ilu); };
+  if (s->graph_uses[j]++ == 0) return step();
   cudaGraph_t g = nullptr;
   E2D_CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-  const int rc = arnoldi_step(h, j, eps0, nm, ilu);
+  const int rc = step();
   const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc || e != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
@@ -1231,6 +1420,7 @@ int gmres(e2d_handle* h, const e2d_nks_params& p, const std::vector<double>& tol
     gmres_cycle_start_kernel<<<1, VT, 0, h->stream>>>(D, s->nrm, s->active, first ? 1 : 0);
     E2D_CK(cudaGetLastError());
     for (int q = 0; q < m; ++q) s->progress_host[q] = -1;
+    if (s->team && (rc = arnoldi_head_step(h, 0, p.epsilon0, nm, use_ilu(p)))) return rc;
     for (int j = 0; j < m; ++j) {
       if ((rc = run_arnoldi(h, j, p.epsilon0, nm, use_ilu(p)))) return rc;
       E2D_CK(cudaEventRecord(s->step_done[j], h->stream));
