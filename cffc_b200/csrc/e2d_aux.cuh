@@ -23,142 +23,202 @@ constexpr int AUX_THREADS = 256;
 constexpr int GHOST_THREADS = 576;
 constexpr double MILLION = 1000000.0;
 
-// One edge-cell of the W or E (vertical) boundary: side 0 = W, 1 = E.
-__device__ void bc_vertical(const Blocks& B, int b, int j, int side) {
-  const int ICl = NG, ICu = B.nci + NG - 1;
-  const int bc = side == 0 ? B.bcw[size_t(b) * B.NCj + j] : B.bce[size_t(b) * B.NCj + j];
-  const int in = side == 0 ? ICl : ICu;           // first interior column
-  const int dir = side == 0 ? -1 : 1;             // towards the ghosts
-  const double* wo = side == 0 ? B.wow : B.woe;
-  switch (bc) {
-    case E2D_BC_NONE: break;
-    case E2D_BC_FIXED:
-      for (int g = 1; g <= NG; ++g) ghost_set(B, b, in + dir * g, j, wo_at(wo, b, B.NCj, j));
-      break;
-    case E2D_BC_REFLECTION: {
-      double nx, ny;
-      if (side == 0) nfaceW(B, b, ICl, j, nx, ny); else nfaceE(B, b, ICu, j, nx, ny);
-      for (int g = 1; g <= NG; ++g)
-        ghost_set(B, b, in + dir * g, j, reflect(ldW(B, b, in - dir * (g - 1), j), nx, ny));
-      break;
-    }
-    case E2D_BC_PERIODIC:
-      for (int g = 1; g <= NG; ++g)
-        ghost_copy(B, b, in + dir * g, j, side == 0 ? ICu - g + 1 : ICl + g - 1, j);
-      break;
-    case E2D_BC_CHARACTERISTIC: {
-      double nx, ny;
-      if (side == 0) nfaceW(B, b, ICl, j, nx, ny); else nfaceE(B, b, ICu, j, nx, ny);
-      ghost_set(B, b, in + dir, j, bc_char_pressure(ldW(B, b, in, j), wo_at(wo, b, B.NCj, j), nx, ny, B.g, B.gm1i));
-      for (int g = 2; g <= NG; ++g) ghost_copy(B, b, in + dir * g, j, in + dir, j);
-      break;
-    }
-    default:  // BC_CONSTANT_EXTRAPOLATION (and the reference's default)
-      for (int g = 1; g <= NG; ++g) ghost_copy(B, b, in + dir * g, j, in, j);
-      break;
+// Outward unit normal of the block edge's face at cell m of edge e (W, E, S,
+// N): nfaceW/E/S/N of the first interior cell.
+__device__ void edge_normal_at(const Blocks& B, int b, int e, int m, double& nx, double& ny) {
+  switch (e) {
+    case 0: nfaceW(B, b, NG, m, nx, ny); break;
+    case 1: nfaceE(B, b, B.nci + NG - 1, m, nx, ny); break;
+    case 2: nfaceS(B, b, m, NG, nx, ny); break;
+    default: nfaceN(B, b, m, B.ncj + NG - 1, nx, ny); break;
   }
+}
+// Cells of a block's four edges laid end to end (W, E: NCj each; S, N: NCi).
+__device__ __forceinline__ int edge_first(const Blocks& B, int e) {
+  return e < 2 ? e * B.NCj : 2 * B.NCj + (e - 2) * B.NCi;
+}
+__device__ __forceinline__ const int* edge_codes(const Blocks& B, int b, int e) {
+  return e < 2 ? (e ? B.bce : B.bcw) + size_t(b) * B.NCj : (e == 2 ? B.bcs : B.bcn) + size_t(b) * B.NCi;
 }
 
-// One edge-cell of the S or N (horizontal) boundary: side 0 = S, 1 = N.
-__device__ void bc_horizontal(const Blocks& B, int b, int i, int side) {
-  const int JCl = NG, JCu = B.ncj + NG - 1;
-  const int bc = side == 0 ? B.bcs[size_t(b) * B.NCi + i] : B.bcn[size_t(b) * B.NCi + i];
-  const int in = side == 0 ? JCl : JCu;
-  const int dir = side == 0 ? -1 : 1;
-  const double* wo = side == 0 ? B.wos : B.won;
-  switch (bc) {
-    case E2D_BC_NONE: break;
-    case E2D_BC_FIXED:
-      for (int g = 1; g <= NG; ++g) ghost_set(B, b, i, in + dir * g, wo_at(wo, b, B.NCi, i));
-      break;
-    case E2D_BC_REFLECTION: {
-      double nx, ny;
-      if (side == 0) nfaceS(B, b, i, JCl, nx, ny); else nfaceN(B, b, i, JCu, nx, ny);
-      for (int g = 1; g <= NG; ++g)
-        ghost_set(B, b, i, in + dir * g, reflect(ldW(B, b, i, in - dir * (g - 1)), nx, ny));
-      break;
+// The boundary condition of cell m of edge e of block b: both ghost layers.
+// One body for the four edges (the ghosts and the interior cells behind the
+// edge lie `st` apart), with the face normal from the handle's table.
+__device__ __forceinline__ void bc_edge(const Blocks& B, int b, int e, int m) {
+  const bool vert = e < 2, hi = e & 1;
+  const int bc = edge_codes(B, b, e)[m];
+  const double2 nrm = B.edge_nrm[size_t(b) * 2 * (B.NCj + B.NCi) + edge_first(B, e) + m];
+  const size_t plane = size_t(B.NCj) * B.NCi;
+  const int nc = vert ? B.nci : B.ncj, in = hi ? nc + NG - 1 : NG;  // interior cells across, the first one
+  const long long st = (hi ? 1ll : -1ll) * (vert ? 1 : B.NCi);
+  const long long o = (long long)(vert ? cell_var(B, b, 0, m, in) : cell_var(B, b, 0, in, m));
+  auto ld = [&](const double* a, long long q, double* v) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = a[q + (long long)(k * plane)];
+  };
+  auto st4 = [&](double* a, long long q, const double* v) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[q + (long long)(k * plane)] = v[k];
+  };
+  auto set = [&](int g, const PState<double>& w) {  // ghost layer g
+    const CState<double> u = U_of_W(w, B.gm1i);
+    const double wv[4] = {w.d, w.u, w.v, w.p}, uv[4] = {u.d, u.mx, u.my, u.E};
+    st4(B.W, o + g * st, wv);
+    st4(B.U, o + g * st, uv);
+  };
+  double v0[4], v1[4];  // the first two interior cells
+  ld(B.W, o, v0);
+  ld(B.W, o - st, v1);
+  if (bc == E2D_BC_NONE) return;
+  const double* wo = vert ? (hi ? B.woe : B.wow) : (hi ? B.won : B.wos);
+  const PState<double> w0{v0[0], v0[1], v0[2], v0[3]};
+  if (bc == E2D_BC_FIXED) {
+    const PState<double> w = wo_at(wo, b, vert ? B.NCj : B.NCi, m);
+#pragma unroll
+    for (int g = 1; g <= NG; ++g) set(g, w);
+  } else if (bc == E2D_BC_REFLECTION) {
+    set(1, reflect(w0, nrm.x, nrm.y));
+    set(2, reflect(PState<double>{v1[0], v1[1], v1[2], v1[3]}, nrm.x, nrm.y));
+  } else if (bc == E2D_BC_CHARACTERISTIC) {
+    const PState<double> w =
+        bc_char_pressure(w0, wo_at(wo, b, vert ? B.NCj : B.NCi, m), nrm.x, nrm.y, B.g, B.gm1i);
+#pragma unroll
+    for (int g = 1; g <= NG; ++g) set(g, w);
+  } else {
+    // copies: the opposite side's interior (periodic), else the first interior
+    // cell (constant extrapolation, the reference's default)
+#pragma unroll
+    for (int g = 1; g <= NG; ++g) {
+      const long long q = bc == E2D_BC_PERIODIC ? o - (nc - g) * st : o;
+      double wv[4], uv[4];
+      ld(B.W, q, wv);
+      ld(B.U, q, uv);
+      st4(B.W, o + g * st, wv);
+      st4(B.U, o + g * st, uv);
     }
-    case E2D_BC_PERIODIC:
-      for (int g = 1; g <= NG; ++g)
-        ghost_copy(B, b, i, in + dir * g, i, side == 0 ? JCu - g + 1 : JCl + g - 1);
-      break;
-    case E2D_BC_CHARACTERISTIC: {
-      double nx, ny;
-      if (side == 0) nfaceS(B, b, i, JCl, nx, ny); else nfaceN(B, b, i, JCu, nx, ny);
-      ghost_set(B, b, i, in + dir, bc_char_pressure(ldW(B, b, i, in), wo_at(wo, b, B.NCi, i), nx, ny, B.g, B.gm1i));
-      for (int g = 2; g <= NG; ++g) ghost_copy(B, b, i, in + dir * g, i, in + dir);
-      break;
-    }
-    default:
-      for (int g = 1; g <= NG; ++g) ghost_copy(B, b, i, in + dir * g, i, in);
-      break;
   }
 }
+static_assert(NG == 2, "two ghost layers");
+
+// Ghost cell q of block b's exchange, from its neighbour across k (W, E, S, N,
+// then the corners): two layers of an edge, a 2 x 2 patch of a corner.
+__device__ __forceinline__ void exchange_cell(const Blocks& B, int b, int q) {
+  const int ICl = NG, ICu = B.nci + NG - 1, JCl = NG, JCu = B.ncj + NG - 1;
+  const int ne = NG * B.ncj, nn = NG * B.nci, nc = NG * NG;
+  int k, r = q;
+  if (r < 2 * ne) { k = r / ne; r %= ne; }
+  else if ((r -= 2 * ne) < 2 * nn) { k = 2 + r / nn; r %= nn; }
+  else { r -= 2 * nn; k = 4 + r / nc; r %= nc; }
+  const int s = B.neigh[b * 8 + k];
+  if (s < 0) return;
+  int i, j, di, dj;
+  const bool wi = (k == 0 || k == 4 || k == 6), ei = (k == 1 || k == 5 || k == 7);
+  const bool sj = (k == 2 || k == 4 || k == 5), nj = (k == 3 || k == 6 || k == 7);
+  int ri, rj;  // position inside the ghost patch
+  if (k < 2) { ri = r % NG; rj = r / NG; }
+  else if (k < 4) { ri = r % B.nci; rj = r / B.nci; }
+  else { ri = r % NG; rj = r / NG; }
+  if (wi) { i = ICl - NG + ri; di = (ICu + 1) - ICl; }
+  else if (ei) { i = ICu + 1 + ri; di = ICl - (ICu + 1); }
+  else { i = ICl + ri; di = 0; }
+  if (sj) { j = JCl - NG + rj; dj = (JCu + 1) - JCl; }
+  else if (nj) { j = JCu + 1 + rj; dj = JCl - (JCu + 1); }
+  else { j = JCl + rj; dj = 0; }
+  const CState<double> u = ldU(B, s, i + di, j + dj);
+  stU(B, b, i, j, u);
+  stW(B, b, i, j, W_of_U(u, B.gm1));
+}
+
+// Per block (bc_flag_kernel, once per handle): BCF_ANY, an edge cell has a
+// boundary condition; BCF_MIXED, an edge has conditions on some of its cells
+// only or on an edge that also exchanges with a neighbour.
+constexpr unsigned BCF_ANY = 1, BCF_MIXED = 2;
 
 // One CTA per block: exchange, then W/E BCs, then S/N BCs (the reference's
-// order; the S/N pass also fills the corner ghosts).  The status word, the
-// 8 neighbours and the block's BC codes are read together up front; a block
-// whose edges all have code BC_NONE (every edge exchanged) stops after the
-// exchange.
+// order; the S/N pass also fills the corner ghosts).
+//
+// Off the corners a condition reads interior cells only, so in a block whose
+// edges have it on all their cells or on none, and no neighbour where they do,
+// everything but the corners is one round of independent items -- exchanged
+// cells and edge cells, each its own thread -- and a second round, after a
+// barrier, applies to the corners the condition that comes last there: W/E on
+// the ghost rows of an S or N edge without one, else S/N on the ghost columns.
+// A mixed block takes exchange, W/E and S/N one after another.
+//
+// Latency bound, by rounds of loads (B200, cold caches): 12 blocks of 32 x 32
+// with walls and characteristic ends 9.1 us a fill against 12.6 in passes of two
+// edges a thread with the normals from the nodes, 256 periodic blocks of 64 x 64
+// 8.9 against 8.6.
 __global__ void __launch_bounds__(GHOST_THREADS, 2) ghost_fill_kernel(Blocks B) {
   const int b = blockIdx.x;
-  const int ICl = NG, ICu = B.nci + NG - 1, JCl = NG, JCu = B.ncj + NG - 1;
-  __shared__ int failed, nb[8];
-  if (threadIdx.x == 0) failed = *(volatile int*)B.status;
-  if (threadIdx.x < 8) nb[threadIdx.x] = B.neigh[b * 8 + threadIdx.x];
-  int bc_here = 0;
-  for (int q = threadIdx.x; q < 2 * (B.NCj + B.NCi); q += blockDim.x) {
-    const int code = q < B.NCj           ? B.bcw[size_t(b) * B.NCj + q]
-                     : q < 2 * B.NCj     ? B.bce[size_t(b) * B.NCj + q - B.NCj]
-                     : q < 2 * B.NCj + B.NCi ? B.bcs[size_t(b) * B.NCi + q - 2 * B.NCj]
-                                         : B.bcn[size_t(b) * B.NCi + q - 2 * B.NCj - B.NCi];
-    bc_here |= code != E2D_BC_NONE;
+  const unsigned flag = B.bcflag[b];
+  if (*(volatile int*)B.status) return;  // uniform: an earlier kernel failed
+  const int total = 2 * NG * (B.nci + B.ncj) + 4 * NG * NG;
+  const bool mixed = flag & BCF_MIXED;
+  const int phases = mixed ? 3 : (flag & BCF_ANY ? 2 : 1);
+  for (int ph = 0; ph < phases; ++ph) {
+    if (ph) __syncthreads();
+    const int items = mixed ? (ph == 0 ? total : (ph == 1 ? 2 * B.NCj : 2 * B.NCi))
+                            : (ph == 0 ? total + (phases > 1 ? 2 * (B.nci + B.ncj) : 0) : 8 * NG);
+    for (int q = threadIdx.x; q < items; q += blockDim.x) {
+      if (ph == 0 && q < total) {
+        exchange_cell(B, b, q);
+        continue;
+      }
+      int e, m;  // edge and its cell
+      if (mixed) {
+        const int n = ph == 1 ? B.NCj : B.NCi;
+        e = (ph == 1 ? 0 : 2) + q / n;
+        m = q % n;
+      } else if (ph == 0) {
+        const int r = q - total, v = 2 * B.ncj;
+        e = r < v ? r / B.ncj : 2 + (r - v) / B.nci;
+        m = NG + (r < v ? r % B.ncj : (r - v) % B.nci);
+      } else {  // corners: four edges, their 2 NG cells in the ghost rows or columns
+        e = q / (2 * NG);
+        m = q % (2 * NG);
+        if (m >= NG) m += (e < 2 ? B.ncj : B.nci);
+      }
+      // W and E along ghost rows only where the S or N edge has no condition
+      if (e < 2 && (m < NG || m >= B.ncj + NG) &&
+          edge_codes(B, b, m < NG ? 2 : 3)[e ? B.nci + NG : NG - 1] != E2D_BC_NONE)
+        continue;
+      bc_edge(B, b, e, m);
+    }
   }
-  const bool any_bc = __syncthreads_or(bc_here);
-  if (failed) return;  // uniform per CTA
-  // exchange: edges (2 layers) and corners (2x2) from the 8 neighbours
-  const int ne = NG * B.ncj, nn = NG * B.nci, nc = NG * NG;
-  const int total = 2 * ne + 2 * nn + 4 * nc;
-  for (int q = threadIdx.x; q < total; q += blockDim.x) {
-    int k, r = q;
-    if (r < 2 * ne) { k = r / ne; r %= ne; }
-    else if ((r -= 2 * ne) < 2 * nn) { k = 2 + r / nn; r %= nn; }
-    else { r -= 2 * nn; k = 4 + r / nc; r %= nc; }
-    const int s = nb[k];
-    if (s < 0) continue;
-    int i, j, di, dj;
-    const bool wi = (k == 0 || k == 4 || k == 6), ei = (k == 1 || k == 5 || k == 7);
-    const bool sj = (k == 2 || k == 4 || k == 5), nj = (k == 3 || k == 6 || k == 7);
-    int ri, rj;  // position inside the ghost patch
-    if (k < 2) { ri = r % NG; rj = r / NG; }
-    else if (k < 4) { ri = r % B.nci; rj = r / B.nci; }
-    else { ri = r % NG; rj = r / NG; }
-    if (wi) { i = ICl - NG + ri; di = (ICu + 1) - ICl; }
-    else if (ei) { i = ICu + 1 + ri; di = ICl - (ICu + 1); }
-    else { i = ICl + ri; di = 0; }
-    if (sj) { j = JCl - NG + rj; dj = (JCu + 1) - JCl; }
-    else if (nj) { j = JCu + 1 + rj; dj = JCl - (JCu + 1); }
-    else { j = JCl + rj; dj = 0; }
-    const CState<double> u = ldU(B, s, i + di, j + dj);
-    stU(B, b, i, j, u);
-    stW(B, b, i, j, W_of_U(u, B.gm1));
+}
+
+// The normals of the edges' faces, for the fills' whole life.
+__global__ void edge_normal_kernel(Blocks B, double2* nrm) {
+  const int per = 2 * (B.NCj + B.NCi);
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)per * B.nblk;
+       t += (long long)gridDim.x * blockDim.x) {
+    const int b = int(t / per), q = int(t % per);
+    const int e = q < 2 * B.NCj ? q / B.NCj : 2 + (q - 2 * B.NCj) / B.NCi;
+    double2 n;
+    edge_normal_at(B, b, e, q - edge_first(B, e), n.x, n.y);
+    nrm[t] = n;
   }
-  if (!any_bc) return;  // uniform: no boundary condition to apply
-  __syncthreads();
-  const bool s_none_w = B.bcs[size_t(b) * B.NCi + ICl - 1] == E2D_BC_NONE;
-  const bool n_none_w = B.bcn[size_t(b) * B.NCi + ICl - 1] == E2D_BC_NONE;
-  const bool s_none_e = B.bcs[size_t(b) * B.NCi + ICu + 1] == E2D_BC_NONE;
-  const bool n_none_e = B.bcn[size_t(b) * B.NCi + ICu + 1] == E2D_BC_NONE;
-  for (int j = threadIdx.x; j < B.NCj; j += blockDim.x) {
-    const bool mid = (j >= JCl && j <= JCu);
-    if (mid || (j < JCl && s_none_w) || (j > JCu && n_none_w)) bc_vertical(B, b, j, 0);
-    if (mid || (j < JCl && s_none_e) || (j > JCu && n_none_e)) bc_vertical(B, b, j, 1);
+}
+
+// The flags of ghost_fill_kernel, one warp per block.
+__global__ void bc_flag_kernel(Blocks B, unsigned char* flags) {
+  const int b = blockIdx.x;
+  bool any = false, mixed = false;
+  for (int e = 0; e < 4; ++e) {
+    const int n = e < 2 ? B.NCj : B.NCi;
+    const int* code = edge_codes(B, b, e);
+    bool some = false, all = true;
+    for (int q = threadIdx.x; q < n; q += 32) {
+      some |= code[q] != E2D_BC_NONE;
+      all &= code[q] != E2D_BC_NONE;
+    }
+    some = __any_sync(0xffffffffu, some);
+    all = __all_sync(0xffffffffu, all);
+    any |= some;
+    mixed |= some && (!all || B.neigh[b * 8 + e] >= 0);
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < B.NCi; i += blockDim.x) {
-    bc_horizontal(B, b, i, 0);
-    bc_horizontal(B, b, i, 1);
-  }
+  if (threadIdx.x == 0) flags[b] = (unsigned char)((any ? BCF_ANY : 0u) | (mixed ? BCF_MIXED : 0u));
 }
 
 // Positive doubles order like their int64 bit patterns.
@@ -292,11 +352,20 @@ __global__ void step_end_kernel(double* hist, int* step, int fused, int ncase) {
 }
 
 cudaError_t launch_ghost_fill(const Blocks& B, cudaStream_t st) {
-  // one thread per exchanged ghost cell where the block allows (the exchange
-  // is a single round of independent loads), at least one CTA of AUX_THREADS
+  // one thread per exchanged ghost cell or edge cell where the block allows (a
+  // single round of independent loads), at least one CTA of AUX_THREADS
   const int cells = 2 * NG * (B.nci + B.ncj) + 4 * NG * NG;
   const int threads = std::min(GHOST_THREADS, std::max(AUX_THREADS, (cells + 31) / 32 * 32));
   ghost_fill_kernel<<<B.nblk, threads, 0, st>>>(B);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_edge_setup(const Blocks& B, unsigned char* flags, double2* nrm, cudaStream_t st) {
+  bc_flag_kernel<<<B.nblk, 32, 0, st>>>(B, flags);
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  const long long n = 2ll * (B.NCj + B.NCi) * B.nblk;
+  edge_normal_kernel<<<int(std::min<long long>((n + 255) / 256, 1184)), 256, 0, st>>>(B, nrm);
   return cudaGetLastError();
 }
 

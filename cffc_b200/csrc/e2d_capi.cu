@@ -802,6 +802,12 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
       cudaMemset(B.dt, 0, sizeof(double) * h->ncell) || cudaMemset(B.status, 0, sizeof(int) * 2) ||
       cudaMemset(h->step, 0, sizeof(int)))
     return fail(E2D_ERR_CUDA, h);
+  unsigned char* flags = nullptr;
+  double2* nrm = nullptr;
+  if ((rc = dalloc(h, &flags, B.nblk)) || (rc = dalloc(h, &nrm, 2 * size_t(NCj + NCi) * B.nblk))) return fail(rc, h);
+  if (launch_edge_setup(B, flags, nrm, h->stream) != cudaSuccess) return fail(E2D_ERR_CUDA, h);
+  B.bcflag = flags;
+  B.edge_nrm = nrm;
   if (sc->n_stage >= 3) {
     if ((rc = dalloc(h, &h->W3, 4 * h->ncell)) || (rc = dalloc(h, &h->U3, 4 * h->ncell))) return fail(rc, h);
     if (cudaMemset(h->W3, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(h->U3, 0, sizeof(double) * 4 * h->ncell))

@@ -41,6 +41,8 @@ struct Blocks {
   int nblk, nci, ncj, NCi, NCj, NNi, NNj;
   const int* neigh;                // [nblk][8]  W E S N SW SE NW NE
   const int *bcw, *bce, *bcs, *bcn;
+  const unsigned char* bcflag;     // [nblk] what the ghost fill needs to know of the codes (BCF_*)
+  const double2* edge_nrm;         // [nblk][2 (NCj + NCi)] face normals along the edges W, E, S, N
   const double *X, *Y;             // nodes
   const double *wow, *woe, *wos, *won;
   double *W, *U, *dUdt;            // cell state (the solution lives in W, U)

@@ -54,6 +54,7 @@ inline void stage_tile(int precision, int* ti, int* tj) {
   else { *ti = fast::tile_i(); *tj = fast::tile_j(); }
 }
 cudaError_t launch_ghost_fill(const Blocks& B, cudaStream_t st);
+cudaError_t launch_edge_setup(const Blocks& B, unsigned char* flags, double2* nrm, cudaStream_t st);
 cudaError_t launch_cfl(const Blocks& B, double* hist, const int* step, cudaStream_t st);
 cudaError_t launch_norms(const Blocks& B, double* part, double* hist, const int* step, cudaStream_t st);
 cudaError_t launch_slot_init(double* hist, const int* step, int offset, int ncase, cudaStream_t st);
