@@ -12,6 +12,7 @@
 #pragma once
 #include "e2d_device.cuh"
 #include "e2d_geom.cuh"
+#include "e2d_pdl.cuh"
 
 #include <algorithm>
 
@@ -152,6 +153,8 @@ constexpr unsigned BCF_ANY = 1, BCF_MIXED = 2;
 __global__ void __launch_bounds__(GHOST_THREADS, 2) ghost_fill_kernel(Blocks B) {
   const int b = blockIdx.x;
   const unsigned flag = B.bcflag[b];
+  pdl_launch_next();
+  pdl_wait();
   if (*(volatile int*)B.status) return;  // uniform: an earlier kernel failed
   const int total = 2 * NG * (B.nci + B.ncj) + 4 * NG * NG;
   const bool mixed = flag & BCF_MIXED;
@@ -340,12 +343,21 @@ __global__ void slot_init_kernel(double* hist, const int* step, int offset, int 
     h[0] = MILLION; h[1] = 0.0; h[2] = 0.0; h[3] = 0.0;
   }
 }
-// End of a step: the fused epilogue summed r^2 into the next slots' L2 entries.
-__global__ void step_end_kernel(double* hist, int* step, int fused, int ncase) {
+// End of a step: the fused epilogue summed r^2 into the next slots' L2 entries;
+// with `init` the slots after those are made ready for the next step's
+// epilogue (slot_init_kernel's work).
+__global__ void step_end_kernel(double* hist, int* step, int fused, int ncase, int init) {
+  pdl_launch_next();
+  pdl_wait();
   if (fused)
     for (int c = threadIdx.x; c < ncase; c += blockDim.x) {
       double* h = hist + 4 * ((*step + 1) * ncase + c);
       h[2] = sqrt(h[2]);
+    }
+  if (init)
+    for (int c = threadIdx.x; c < ncase; c += blockDim.x) {
+      double* h = hist + 4 * ((*step + 2) * ncase + c);
+      h[0] = MILLION; h[1] = 0.0; h[2] = 0.0; h[3] = 0.0;
     }
   __syncthreads();
   if (threadIdx.x == 0) *step += 1;
@@ -356,8 +368,7 @@ cudaError_t launch_ghost_fill(const Blocks& B, cudaStream_t st) {
   // single round of independent loads), at least one CTA of AUX_THREADS
   const int cells = 2 * NG * (B.nci + B.ncj) + 4 * NG * NG;
   const int threads = std::min(GHOST_THREADS, std::max(AUX_THREADS, (cells + 31) / 32 * 32));
-  ghost_fill_kernel<<<B.nblk, threads, 0, st>>>(B);
-  return cudaGetLastError();
+  return launch_pdl(ghost_fill_kernel, B.nblk, threads, 0, st, B);
 }
 
 cudaError_t launch_edge_setup(const Blocks& B, unsigned char* flags, double2* nrm, cudaStream_t st) {
@@ -384,9 +395,8 @@ cudaError_t launch_slot_init(double* hist, const int* step, int offset, int ncas
   slot_init_kernel<<<1, 128, 0, st>>>(hist, step, offset, ncase);
   return cudaGetLastError();
 }
-cudaError_t launch_step_end(double* hist, int* step, int fused, int ncase, cudaStream_t st) {
-  step_end_kernel<<<1, 128, 0, st>>>(hist, step, fused, ncase);
-  return cudaGetLastError();
+cudaError_t launch_step_end(double* hist, int* step, int fused, int ncase, int init, cudaStream_t st) {
+  return launch_pdl(step_end_kernel, 1, 128, 0, st, hist, step, fused, ncase, init);
 }
 cudaError_t launch_fill(double* p, long long n, double v, cudaStream_t st) {
   int grid = int((n + 255) / 256);

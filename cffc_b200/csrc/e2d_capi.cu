@@ -485,6 +485,11 @@ int ensure_recon(e2d_handle* h) {
   return 0;
 }
 
+void drop_step_graphs(e2d_handle* h) {
+  for (auto& g : h->step_graph)
+    if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+}
+
 int ensure_hist(e2d_handle* h, int n) {
   if (n <= h->hist_cap) return 0;
   int cap = n < 64 ? 64 : n;
@@ -498,17 +503,19 @@ int ensure_hist(e2d_handle* h, int n) {
   }
   h->hist = p;
   h->hist_cap = cap;
-  if (h->step_graph) { cudaGraphExecDestroy(h->step_graph); h->step_graph = nullptr; }
+  drop_step_graphs(h);
   return 0;
 }
 
 // CFL + global minimum and the residual norms of the current state into the
 // current step's history slot: the head of the reference's explicit step
 // (Euler2DQuadSolvers.cc:657-696).  Needed before the first step only; every
-// step's last stage computes them for the following step.
+// step's last stage computes them for the following step, into a slot made
+// ready here for the first step and by each step's end for the next.
 cudaError_t enqueue_step_head(e2d_handle* h) {
   cudaError_t e;
   if ((e = launch_slot_init(h->hist, h->step, 0, h->B.ncase, h->stream))) return e;
+  if (h->sc.rs_epsilon <= 0.0 && (e = launch_slot_init(h->hist, h->step, 1, h->B.ncase, h->stream))) return e;
   if ((e = launch_cfl(h->B, h->hist, h->step, h->stream))) return e;
   return launch_norms(h->B, h->part, h->hist, h->step, h->stream);
 }
@@ -592,7 +599,6 @@ cudaError_t enqueue_step(e2d_handle* h) {
   cudaError_t e;
   const bool smooth = h->sc.rs_epsilon > 0.0;
   if (smooth && (e = enqueue_step_head(h))) return e;
-  if ((e = launch_slot_init(h->hist, h->step, 1, h->B.ncase, h->stream))) return e;
   if ((e = launch_freeze_check(h))) return e;
   for (int stage = 1; stage <= h->sc.n_stage; ++stage) {
     if ((e = ghost_fill_for(h, stage))) return e;
@@ -602,7 +608,7 @@ cudaError_t enqueue_step(e2d_handle* h) {
       return e;
     }
   }
-  return launch_step_end(h->hist, h->step, smooth ? 0 : 1, h->B.ncase, h->stream);
+  return launch_step_end(h->hist, h->step, smooth ? 0 : 1, h->B.ncase, smooth ? 0 : 1, h->stream);
 }
 
 }  // namespace e2d_host
@@ -922,7 +928,7 @@ void e2d_destroy(e2d_handle* h) {
   }
   cudaSetDevice(h->device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  if (h->step_graph) cudaGraphExecDestroy(h->step_graph);
+  drop_step_graphs(h);
   nks_free(h);
   for (void* p : h->allocs) cudaFree(p);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -1102,17 +1108,20 @@ int e2d_rk_steps(e2d_handle* h, int n_steps, double* hist) {
   }
   if (n_steps == 0) return 0;
   CK(cudaSetDevice(h->device));
-  int rc = ensure_hist(h, n_steps + 1);  // the last step fills slot n_steps
+  int rc = ensure_hist(h, n_steps + 2);  // the last step fills slot n_steps and clears the one after it
   if (rc) return rc;
   // the stage kernels do not write the optional reconstruction arrays
   const Blocks saved = h->B;
   h->B.dWdx = h->B.dWdy = h->B.phi = nullptr;
   CK(cudaMemsetAsync(h->step, 0, sizeof(int), h->stream));
   CK(enqueue_step_head(h));
-  if (!h->step_graph) {
+  // one graph of a step and, for long runs, one of STEP_GROUP steps
+  for (int k = 0; k < 2; ++k) {
+    if (h->step_graph[k] || (k == 1 && n_steps < STEP_GROUP_MIN)) continue;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = enqueue_step(h);
+    cudaError_t e = cudaSuccess;
+    for (int s = 0; s < (k ? STEP_GROUP : 1) && e == cudaSuccess; ++s) e = enqueue_step(h);
     cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
     if (e != cudaSuccess || e2 != cudaSuccess) {
       if (g) cudaGraphDestroy(g);
@@ -1120,12 +1129,15 @@ int e2d_rk_steps(e2d_handle* h, int n_steps, double* hist) {
       fprintf(stderr, "cffc_e2d: step capture failed: %s\n", cudaGetErrorString(e ? e : e2));
       return E2D_ERR_CUDA;
     }
-    e = cudaGraphInstantiate(&h->step_graph, g, 0);
+    e = cudaGraphInstantiate(&h->step_graph[k], g, 0);
     cudaGraphDestroy(g);
-    if (e != cudaSuccess) { h->B = saved; h->step_graph = nullptr; return E2D_ERR_CUDA; }
+    if (e != cudaSuccess) { h->B = saved; h->step_graph[k] = nullptr; return E2D_ERR_CUDA; }
   }
   h->B = saved;
-  for (int s = 0; s < n_steps; ++s) CK(cudaGraphLaunch(h->step_graph, h->stream));
+  int s = 0;
+  if (h->step_graph[1] && n_steps >= STEP_GROUP_MIN)
+    for (; s + STEP_GROUP <= n_steps; s += STEP_GROUP) CK(cudaGraphLaunch(h->step_graph[1], h->stream));
+  for (; s < n_steps; ++s) CK(cudaGraphLaunch(h->step_graph[0], h->stream));
   if (h->sc.n_stage >= 2) {
     // The reference keeps one state array, so after a multistage step its
     // ghost cells hold the last stage's exchange and BCs; here those went
@@ -1207,10 +1219,7 @@ int e2d_set_precision(e2d_handle* h, int precision) {
   h->sc.precision = precision;
   apply_selection(h);
   // captured launches hold the previous precision's kernels
-  if (h->step_graph) {
-    cudaGraphExecDestroy(h->step_graph);
-    h->step_graph = nullptr;
-  }
+  drop_step_graphs(h);
   nks_drop_graphs(h);
   return 0;
 }
@@ -1289,7 +1298,7 @@ int e2d_kernel_times(e2d_handle* h, int n_steps, double out[6]) {
       CK(launch_explicit_stage(h, 2, 1));
       CK(cudaEventRecord(ev[6], h->stream));
     }
-    CK(launch_step_end(h->hist, h->step, 1, h->B.ncase, h->stream));
+    CK(launch_step_end(h->hist, h->step, 1, h->B.ncase, 0, h->stream));
     CK(cudaEventRecord(ev[7], h->stream));
     CK(cudaEventSynchronize(ev[7]));
     float t[8] = {0};

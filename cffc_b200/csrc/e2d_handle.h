@@ -64,8 +64,8 @@ struct e2d_handle {
   bool sel_march[3] = {false, false, false};
   int sel_rows[3] = {7, 7, 7};
   double sel_us[3] = {0.0, 0.0, 0.0};
-  // captured explicit step
-  cudaGraphExec_t step_graph = nullptr;
+  // captured explicit steps: one, STEP_GROUP of them
+  cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
   e2d_nks_state* nks = nullptr;
 };
 
@@ -79,6 +79,13 @@ struct e2d_handle {
   } while (0)
 
 namespace e2d_host {
+
+// Explicit steps per launched graph in runs of STEP_GROUP_MIN steps and more: a
+// graph launch costs the device a gap of about 1.7 us (100 steps of 16 blocks
+// of 32 x 32: 2.75 ms one by one, 2.57 in fours, 2.59 in tens), capturing and
+// instantiating the second graph costs a handle's first run about 100 us, so
+// shorter runs launch step by step.
+constexpr int STEP_GROUP = 4, STEP_GROUP_MIN = 64;
 
 template <class T> int dalloc(e2d_handle* h, T** p, size_t n) {
   void* q = nullptr;

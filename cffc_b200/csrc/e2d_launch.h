@@ -58,6 +58,6 @@ cudaError_t launch_edge_setup(const Blocks& B, unsigned char* flags, double2* nr
 cudaError_t launch_cfl(const Blocks& B, double* hist, const int* step, cudaStream_t st);
 cudaError_t launch_norms(const Blocks& B, double* part, double* hist, const int* step, cudaStream_t st);
 cudaError_t launch_slot_init(double* hist, const int* step, int offset, int ncase, cudaStream_t st);
-cudaError_t launch_step_end(double* hist, int* step, int fused, int ncase, cudaStream_t st);
+cudaError_t launch_step_end(double* hist, int* step, int fused, int ncase, int init, cudaStream_t st);
 cudaError_t launch_fill(double* p, long long n, double v, cudaStream_t st);
 }  // namespace e2d

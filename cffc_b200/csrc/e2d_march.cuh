@@ -48,6 +48,7 @@
 // stage_kernel covers the other block sets.
 #pragma once
 #include "e2d_march_args.h"
+#include "e2d_pdl.cuh"
 #include "e2d_tc.cuh"
 
 namespace e2d {
@@ -674,25 +675,40 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
   const Blocks& B = a.B;
   const int tid = threadIdx.x;
   const long long g0 = m.nchunk * blockIdx.x / gridDim.x, g1 = m.nchunk * (blockIdx.x + 1) / gridDim.x;
-  if (tid == 0) {
-    s.failed = *(volatile int*)B.status;
-    tc::mbar_init(&s.full[0], 1);
-    tc::mbar_init(&s.full[1], 1);
-    tc::mbar_init(&s.fullu, 1);
-  }
-  __syncthreads();
-  if (s.failed || g0 >= g1) return;  // an earlier kernel failed: stop marching (uniform)
   const size_t plane = size_t(B.NCi) * B.NCj;
 
-  auto issue = [&](long long gg, int buf) {
-    const Chunk k = decode(m, gg);
+  // the window of chunk gg: the geometry and nodes, the state
+  auto issue_geo = [&](const Chunk& k, int buf) {
     uint64_t* bar = &s.full[buf];
     expect_tx(bar, TILE_BYTES);
-    tma3(&s.in[buf].W[0][0][0], &m.tmW, bar, k.i0, k.j0, 4 * k.b);
     tma3(&s.in[buf].G[0][0][0], &m.tmG, bar, k.i0, k.j0, GEOM_NF * k.b);
     tma3(&s.in[buf].N[0][0][0], &m.tmN, bar, k.i0, k.j0, 2 * k.b);
   };
-  if (tid == 0) issue(g0, 0);
+  auto issue_state = [&](const Chunk& k, int buf) {
+    tma3(&s.in[buf].W[0][0][0], &m.tmW, &s.full[buf], k.i0, k.j0, 4 * k.b);
+  };
+  auto issue = [&](long long gg, int buf) {
+    const Chunk k = decode(m, gg);
+    issue_state(k, buf);
+    issue_geo(k, buf);
+  };
+  // the first chunk's geometry before anything the stream computes (pdl_wait)
+  if (tid == 0) {
+    tc::mbar_init(&s.full[0], 1);
+    tc::mbar_init(&s.full[1], 1);
+    tc::mbar_init(&s.fullu, 1);
+    if (g0 < g1) issue_geo(decode(m, g0), 0);
+  }
+  pdl_wait();
+  if (tid == 0) {
+    s.failed = *(volatile int*)B.status;
+    if (g0 < g1) issue_state(decode(m, g0), 0);
+  }
+  __syncthreads();
+  if (s.failed || g0 >= g1) {  // an earlier kernel failed: stop marching (uniform), the copies landed
+    if (tid == 0 && g0 < g1) tc::mbar_wait(&s.full[0], 0u, WAIT_ITERS);
+    return;
+  }
   // update inputs by TMA (explicit stages whose arrays have tensor maps)
   const bool upd = UPD && (MODE == 1 || MODE == 2) && m.upd;
 #if E2D_MARCH_UPD
@@ -834,6 +850,12 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
       issue(gg + 1, 0);
     }
   }
+  // The next kernel may start beside the last update where CTAs march over
+  // several chunks and end at different times; started that early in a launch
+  // of one chunk a CTA its waiting CTAs cost more than they hide (100 two-stage
+  // steps: 1M cells 3.08 ms, against 3.15 started at the kernel's begin or not
+  // at all; 16 blocks of 32 x 32 2.45 ms so, 2.30 at the CTAs' end).
+  if (m.nchunk > gridDim.x) pdl_launch_next();
   // the last chunk's update
   if (pcase >= 0) {
     if (FUSE && pcase != cur_case) {
@@ -876,8 +898,7 @@ cudaError_t march_one(const MarchArgs& m, int grid, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  mk::march_kernel<MODE, FUSE, ROE><<<grid, mk::THREADS, march_smem_bytes(), st>>>(m);
-  return cudaGetLastError();
+  return launch_pdl(mk::march_kernel<MODE, FUSE, ROE>, grid, mk::THREADS, march_smem_bytes(), st, m);
 }
 // grid: CTAs of the persistent launch (the caller sizes it to the SMs)
 template <bool ROE>

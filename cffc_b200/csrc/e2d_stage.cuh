@@ -23,6 +23,7 @@
 // the CFL step and the norms stay FP64).  E2D_NS names the namespace.
 #pragma once
 #include "e2d_device.cuh"
+#include "e2d_pdl.cuh"
 
 #ifndef E2D_NS
 #error "E2D_NS must name the kernel namespace"
@@ -288,6 +289,14 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   const int t = blockIdx.x % tiles;
   const int i0 = (t % a.tiles_i) * TI;   // interior index of the tile's first cell
   const int j0 = (t / a.tiles_i) * TJ;   // == array index of the halo origin
+  // the nodes before anything the stream computes (pdl_wait)
+  for (int q = tid; q < NJ * NI; q += NTHREADS) {
+    const int nj = q / NI, ni = q % NI, I = i0 + ni, J = j0 + nj;
+    const bool in = I < B.NNi && J < B.NNj;
+    s.X[nj][ni] = in ? B.X[node_ix(B, b, J, I)] : 0.0;
+    s.Y[nj][ni] = in ? B.Y[node_ix(B, b, J, I)] : 0.0;
+  }
+  pdl_wait();
   __shared__ int failed, frozen;
   if (tid == 0) {
     failed = *(volatile int*)B.status;
@@ -300,17 +309,11 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   const double* dtmin_p = a.hist ? a.hist + 4 * ((*a.step) * B.ncase + cs) : nullptr;
   const double g = B.g, gm1 = B.gm1, gm1i = B.gm1i;
 
-  // ---- stage W and nodes (halo tile) --------------------------------------
+  // ---- stage W (halo tile) --------------------------------------
   for (int q = tid; q < 4 * HJ * HI; q += NTHREADS) {
     const int v = q / (HJ * HI), r = q % (HJ * HI), hj = r / HI, hi = r % HI;
     const int I = i0 + hi, J = j0 + hj;
     s.W[v][hj][hi] = RT((I < B.NCi && J < B.NCj) ? a.Win[cell_var(B, b, v, J, I)] : 0.0);
-  }
-  for (int q = tid; q < NJ * NI; q += NTHREADS) {
-    const int nj = q / NI, ni = q % NI, I = i0 + ni, J = j0 + nj;
-    const bool in = I < B.NNi && J < B.NNj;
-    s.X[nj][ni] = in ? B.X[node_ix(B, b, J, I)] : 0.0;
-    s.Y[nj][ni] = in ? B.Y[node_ix(B, b, J, I)] : 0.0;
   }
   __syncthreads();
 
@@ -647,8 +650,7 @@ cudaError_t launch_one(const StageArgs& a, cudaStream_t st) {
     configured = true;
   }
   const int grid = a.B.nblk * a.tiles_i * a.tiles_j;
-  stage_kernel<MODE, FUSE, ROE><<<grid, NTHREADS, sizeof(Smem), st>>>(a);
-  return cudaGetLastError();
+  return launch_pdl(stage_kernel<MODE, FUSE, ROE>, grid, NTHREADS, sizeof(Smem), st, a);
 }
 template <bool ROE>
 cudaError_t launch_flux(const StageArgs& a, cudaStream_t st) {
