@@ -18,8 +18,10 @@
 // them, issue active 46 %), and the pair's exchange between layers; the next
 // weights arrive (cp.async.bulk) under it.  Measured against a kernel per
 // layer with activations in HBM and 4 warps per SM (B200): prediction of 300,007
-// rows 2,005 -> 593 us, a training step on 8,192 rows 753 -> 105 us
-// (net_kernel 46, dw_kernel 34, adam_kernel 7).  Swizzled operand tiles were
+// rows 2,005 -> 593 us, a training step on 8,192 rows 753 -> 94 us
+// (net_kernel 46, dw_kernel 34, adam_kernel 7; 105 us before the kernels of a
+// step were programmatic dependents of one another and read the minibatch's
+// rows from host memory instead of after a copy).  Swizzled operand tiles were
 // measured too (no faster: the products are not the bound; their strided
 // writes to the peer cost 10 %).
 //
@@ -40,6 +42,7 @@
 #include <vector>
 
 #include "../../include/cffc_e2d.h"
+#include "e2d_pdl.cuh"
 #include "e2d_tc.cuh"
 
 using namespace e2d;
@@ -125,7 +128,7 @@ __device__ __forceinline__ float4 ld4(const float* p, int vec) {
 struct NetArgs {
   const float *X, *T;         // [*][16], [*][4]
   int vec;                    // X, T and Y are 16-byte aligned
-  const int* idx;             // rows of the pass (null: 0 .. n-1)
+  const int* idx;             // rows of the pass, in host memory (null: 0 .. n-1)
   int n;
   float inv_n;
   const uint16_t *wk, *wt;    // BF16 weights and transposes, canonical tiles at the parameter offsets
@@ -144,6 +147,7 @@ struct NetSmem {
   uint8_t W0[HALF * DF * 2], W4[DO * DH * 2], W4T[HALF * DO * 2];
   uint8_t X[TILE * DF * 2], dY[TILE * DO * 2];
   float b[DNL][HALF], b4[DO];
+  int idx[TILE];                  // rows of the tile
   double lw[4];
   uint64_t bar, wbar;
   uint32_t taddr;
@@ -157,6 +161,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) net_kernel(co
   const uint32_t rank = tc::cluster_rank();
   const int cluster = blockIdx.x >> 1, nclusters = gridDim.x >> 1;
   const int ntiles = (a.n + TILE - 1) / TILE;
+  // what depends on no earlier kernel: barriers, TMEM, the first tile's rows
+  if (tid == 0) {
+    tc::mbar_init(&s.bar, 1);
+    tc::mbar_init(&s.wbar, 1);
+  }
+  if (warp == 0) tc::tmem_alloc(&s.taddr, 256);
+  auto row_of = [&](int tile) {
+    const int g = tile * TILE + tid;
+    return tid < TILE && g < a.n ? (a.idx ? a.idx[g] : g) : 0;
+  };
+  int next_row = row_of(cluster);
+  pdl_wait();
   // constant operands (16 bytes a thread) and biases
   auto copy = [&](uint8_t* dst, const uint16_t* src, int bytes) {
     for (int q = tid; q < bytes / 16; q += NT) reinterpret_cast<uint4*>(dst)[q] = reinterpret_cast<const uint4*>(src)[q];
@@ -167,11 +183,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) net_kernel(co
   if (tid < HALF)
     for (int l = 0; l < DNL; ++l) s.b[l][tid] = a.p[b_off(l) + rank * HALF + tid];
   if (tid < DO) s.b4[tid] = a.p[b_off(DNL) + tid];
-  if (tid == 0) {
-    tc::mbar_init(&s.bar, 1);
-    tc::mbar_init(&s.wbar, 1);
-  }
-  if (warp == 0) tc::tmem_alloc(&s.taddr, 256);
   cta_sync_async();
   tc::cluster_sync();  // the peer runs: its shared memory may be written
   const uint32_t tm = s.taddr, td = tm, ty = tm + HALF;  // hidden products, outputs
@@ -229,11 +240,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) net_kernel(co
   for (int tile = cluster; tile < ntiles; tile += nclusters) {
     const int grow = tile * TILE + row;
     const bool valid = grow < a.n, more = tile + nclusters < ntiles;
+    if (tid < TILE) s.idx[tid] = next_row;
+    if (more) next_row = row_of(tile + nclusters);
+    __syncthreads();
     if (tid < 2 * TILE) {  // X: 8 features a thread
       const int r = tid & (TILE - 1), c = tid >> 7, g = tile * TILE + r;
       float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (g < a.n) {
-        const float* x = a.X + size_t(a.idx ? a.idx[g] : g) * DF + 8 * c;
+        const float* x = a.X + size_t(s.idx[r]) * DF + 8 * c;
         const float4 x0 = ld4(x, a.vec), x1 = ld4(x + 4, a.vec);
         v[0] = x0.x; v[1] = x0.y; v[2] = x0.z; v[3] = x0.w; v[4] = x1.x; v[5] = x1.y; v[6] = x1.z; v[7] = x1.w;
       }
@@ -310,7 +324,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NT, 1) net_kernel(co
 #pragma unroll
       for (int q = 0; q < 16; ++q) d[q] = 0.0f;
       if (valid) {
-        const float4 t = ld4(a.T + size_t(a.idx ? a.idx[grow] : grow) * DO_USED, a.vec);
+        const float4 t = ld4(a.T + size_t(s.idx[row]) * DO_USED, a.vec);
         const float tq[4] = {t.x, t.y, t.z, t.w};
 #pragma unroll
         for (int q = 0; q < DO_USED; ++q) {
@@ -455,6 +469,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_kernel(const __grid_constant
   DwSmem& s = *reinterpret_cast<DwSmem*>(smraw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, item = blockIdx.x;
   if (item >= DW_ITEMS) {
+    pdl_wait();
     bias_piece(a, item - DW_ITEMS, reinterpret_cast<float*>(smraw));
     return;
   }
@@ -478,6 +493,7 @@ __global__ void __launch_bounds__(DW_THREADS, 1) dw_kernel(const __grid_constant
     s.failed = 0;
   }
   if (warp == 0) tc::tmem_alloc(&s.taddr, DWB * DWN);
+  pdl_wait();
   cta_sync_async();
   const uint32_t tm = s.taddr;
   const int nchunk = (a.n + RC - 1) / RC, per = a.rows / RC, ngroup = (nchunk + per - 1) / per;
@@ -578,10 +594,11 @@ __global__ void cast_kernel(const float* __restrict__ p, uint16_t* wk, uint16_t*
 
 // Adam (Kingma & Ba, 2015), the BF16 copies of the new weights, and the
 // step's loss from the clusters' sums.
-__global__ void adam_kernel(float* p, const float* __restrict__ g, float* m, float* v, float lr, float b1, float b2,
+__global__ void adam_kernel(float* p, const float* g, float* m, float* v, float lr, float b1, float b2,
                             float eps, float c1, float c2, uint16_t* wk, uint16_t* wt, const double* lpart, int nl,
                             double rows, float* loss) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
   if (q < NPARAM) {
     const float gq = g[q];
     const float mq = b1 * m[q] + (1.0f - b1) * gq;
@@ -610,7 +627,10 @@ struct Pcg {
   double uniform() { return (next() + 0.5) / 4294967296.0; }
 };
 
-constexpr int IDX_RING = 4;  // minibatch row lists on their way to the device
+// Minibatch row lists in pinned host memory, read from there by net_kernel
+// (512 bytes a CTA, before it waits for the step before; a copy to the device
+// would stand between two steps' kernels), reused in two halves.
+constexpr int IDX_RING = 8, IDX_HALF = IDX_RING / 2;
 
 }  // namespace
 
@@ -625,9 +645,8 @@ struct e2d_mlp_deep {
   uint16_t* dz[DNL] = {};                      // deltas of the hidden layers, [cap][256] tiles
   float* gp = nullptr;                         // [CTAs][4][128 x 128] GELU' of the tiles in work
   double* lpart = nullptr;                     // [clusters] loss sums
-  int* idx[IDX_RING] = {};                     // [icap] minibatch rows
-  int* hidx[IDX_RING] = {};                    // their pinned host copies
-  cudaEvent_t sent[IDX_RING] = {};             // the copy out of hidx is done
+  int* hidx = nullptr;                         // [IDX_RING][icap] minibatch rows (pinned host memory)
+  cudaEvent_t read[2] = {};                    // the steps that read a half of hidx are done
   float* loss = nullptr;                       // [hcap] loss history of a training call
   int* err = nullptr;
   void* ws = nullptr;                          // the work arrays' memory (rebuilt on growth)
@@ -672,12 +691,11 @@ int ensure_cap(e2d_mlp_deep* d, int rows) {
 }
 
 void free_train(e2d_mlp_deep* d) {
-  for (int k = 0; k < IDX_RING; ++k) {
-    if (d->idx[k]) cudaFree(d->idx[k]);
-    if (d->hidx[k]) cudaFreeHost(d->hidx[k]);
-    if (d->sent[k]) cudaEventDestroy(d->sent[k]);
-    d->idx[k] = d->hidx[k] = nullptr;
-    d->sent[k] = nullptr;
+  if (d->hidx) cudaFreeHost(d->hidx);
+  d->hidx = nullptr;
+  for (auto& e : d->read) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
   }
   if (d->loss) cudaFree(d->loss);
   d->loss = nullptr;
@@ -691,10 +709,9 @@ int ensure_train(e2d_mlp_deep* d, int batch, int steps) {
   if (steps < d->hcap) steps = d->hcap;
   free_train(d);
   bool ok = cudaMalloc(&d->loss, sizeof(float) * size_t(steps > 0 ? steps : 1)) == cudaSuccess;
-  for (int k = 0; k < IDX_RING && ok; ++k)
-    ok = cudaMalloc(&d->idx[k], sizeof(int) * size_t(batch)) == cudaSuccess &&
-         cudaMallocHost(&d->hidx[k], sizeof(int) * size_t(batch)) == cudaSuccess &&
-         cudaEventCreateWithFlags(&d->sent[k], cudaEventDisableTiming) == cudaSuccess;
+  ok = ok && cudaMallocHost(&d->hidx, sizeof(int) * size_t(batch) * IDX_RING) == cudaSuccess;
+  for (int k = 0; k < 2 && ok; ++k)
+    ok = cudaEventCreateWithFlags(&d->read[k], cudaEventDisableTiming) == cudaSuccess;
   if (!ok) {
     free_train(d);
     return E2D_ERR_NOMEM;
@@ -724,8 +741,9 @@ NetArgs net_args(const e2d_mlp_deep* d, const float* X, const float* T, const in
 // rows are grouped as one group per SM, so that the sums' order depends on n
 // alone.
 int gradient_rows(e2d_mlp_deep* d, const float* X, const float* T, const int* idx, int n, cudaStream_t st) {
-  net_kernel<true><<<net_grid(d, n), NT, sizeof(NetSmem), st>>>(net_args(d, X, T, idx, n, nullptr));
-  if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
+  if (launch_pdl(net_kernel<true>, net_grid(d, n), NT, sizeof(NetSmem), st, net_args(d, X, T, idx, n, nullptr)) !=
+      cudaSuccess)
+    return E2D_ERR_CUDA;
   DwArgs w{};
   w.xb = d->xb; w.dy = d->dy;
   for (int l = 0; l < DNL; ++l) { w.act[l] = d->act[l]; w.dz[l] = d->dz[l]; }
@@ -734,8 +752,8 @@ int gradient_rows(e2d_mlp_deep* d, const float* X, const float* T, const int* id
   w.rows = (w.brows + RC - 1) / RC * RC;
   w.g = d->g;
   w.err = d->err;
-  dw_kernel<<<DW_ITEMS + DW_BIAS, DW_THREADS, sizeof(DwSmem), st>>>(w);
-  return cudaGetLastError() == cudaSuccess ? 0 : E2D_ERR_CUDA;
+  return launch_pdl(dw_kernel, DW_ITEMS + DW_BIAS, DW_THREADS, sizeof(DwSmem), st, w) == cudaSuccess ? 0
+                                                                                                      : E2D_ERR_CUDA;
 }
 
 int check_err(e2d_mlp_deep* d, cudaStream_t st) {
@@ -869,10 +887,10 @@ int e2d_mlp_deep_train(e2d_mlp_deep* d, const float* X, const float* T, int n, i
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const int nl = net_grid(d, b) / 2;
   for (int k = 0; k < steps; ++k) {
-    const int slot = k % IDX_RING;
-    // the list's last copy to the device is done (an earlier call's included)
-    if (cudaEventSynchronize(d->sent[slot]) != cudaSuccess) return E2D_ERR_CUDA;
-    int* hidx = d->hidx[slot];
+    const int slot = k % IDX_RING, half = slot / IDX_HALF;
+    // the half's last readers are done (an earlier call's included)
+    if (slot % IDX_HALF == 0 && cudaEventSynchronize(d->read[half]) != cudaSuccess) return E2D_ERR_CUDA;
+    int* hidx = d->hidx + size_t(slot) * d->icap;
     for (int q = 0; q < b;) {
       if (pos >= n) {  // Fisher-Yates shuffle of the rows per epoch
         for (int i = n - 1; i > 0; --i) std::swap(perm[i], perm[int(rng.next() % uint32_t(i + 1))]);
@@ -883,15 +901,13 @@ int e2d_mlp_deep_train(e2d_mlp_deep* d, const float* X, const float* T, int n, i
       q += take;
       pos += take;
     }
-    if (cudaMemcpyAsync(d->idx[slot], hidx, sizeof(int) * b, cudaMemcpyHostToDevice, st) != cudaSuccess ||
-        cudaEventRecord(d->sent[slot], st) != cudaSuccess)
-      return E2D_ERR_CUDA;
-    if ((rc = gradient_rows(d, X, T, d->idx[slot], b, st))) return rc;
+    if ((rc = gradient_rows(d, X, T, hidx, b, st))) return rc;
     ++d->adam_t;
     const float c1 = 1.0f - powf(b1, float(d->adam_t)), c2 = 1.0f - powf(b2, float(d->adam_t));
-    adam_kernel<<<(NPARAM + 255) / 256, 256, 0, st>>>(d->p, d->g, d->m, d->v, lr, b1, b2, eps, c1, c2, d->wk, d->wt,
-                                                      d->lpart, nl, double(b), loss_hist ? d->loss + k : nullptr);
-    if (cudaGetLastError() != cudaSuccess) return E2D_ERR_CUDA;
+    if (launch_pdl(adam_kernel, (NPARAM + 255) / 256, 256, 0, st, d->p, d->g, d->m, d->v, lr, b1, b2, eps, c1, c2, d->wk,
+                   d->wt, d->lpart, nl, double(b), loss_hist ? d->loss + k : nullptr) != cudaSuccess ||
+        ((slot % IDX_HALF == IDX_HALF - 1 || k == steps - 1) && cudaEventRecord(d->read[half], st) != cudaSuccess))
+      return E2D_ERR_CUDA;
   }
   if (loss_hist && steps > 0 &&
       cudaMemcpyAsync(loss_hist, d->loss, sizeof(float) * size_t(steps), cudaMemcpyDeviceToHost, st) != cudaSuccess)
