@@ -142,8 +142,8 @@ void stage_buffers(e2d_handle* h, int k, double*& W, double*& U) {
 }
 
 // The stage kernel for a stage: the column-marching kernel where the handle
-// allows it (even block width, no degenerate edges) and the autotuner chose
-// it, else the tiled stage kernel.
+// allows it (no degenerate edges; odd widths in exact precision only) and the
+// autotuner chose it, else the tiled stage kernel.
 cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
   if (h->march) {
     const bool ex = h->sc.precision == E2D_PREC_FP64_EXACT;
@@ -151,11 +151,13 @@ cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
     if (a.Win == h->B.W) tw = &h->tmW[0];
     else if (a.Win == h->B.W2) tw = &h->tmW[1];
     else if (a.Win == h->W3 && h->W3) tw = &h->tmW[2];
-    if (tw) {
+    const bool plain = h->march_plain;
+    if (tw || plain) {
       MarchArgs m;
       memset(&m, 0, sizeof(m));
       m.a = a;
-      m.tmW = *tw;
+      m.plain = plain;
+      if (!plain) m.tmW = *tw;
       m.tmG = ex ? h->tmGx : h->tmG;
       m.tmN = h->tmN;
       m.geom = ex ? h->geomx : h->geom;
@@ -225,51 +227,58 @@ bool encode3(CUtensorMap* map, void* base, uint64_t d0, uint64_t d1, uint64_t d2
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Geometry, padded nodes and tensor maps of the marching kernel.  The handle
-// keeps the tiled stage kernel when the marching kernel does not apply: an
-// odd block width (row strides of the tensor maps must be multiples of 16
-// bytes) or a degenerate edge.
+// Geometry, padded nodes and tensor maps of the marching kernel; no maps for
+// an odd block width (their row strides must be multiples of 16 bytes), whose
+// windows the exact build copies itself.  The handle keeps the tiled stage
+// kernel when the marching kernel does not apply: a degenerate edge, an odd
+// width in the fast precisions.
 int setup_march(e2d_handle* h) {
   h->march = h->march_ok = false;
   const Blocks& B = h->B;
-  if (B.NCi % 2 || !encode_fn()) return 0;
+  h->march_plain = B.NCi % 2 != 0;
+  if (!h->march_plain && !encode_fn()) return 0;
   const int mi = fast::march_strip_cols(), wj = fast::march_window_rows();
   const int NNp = B.NNi + 1;  // NNi is odd for an even NCi
   int rc;
   int* degenerate = nullptr;
-  if ((rc = dalloc(h, &h->geom, size_t(GEOM_NF) * h->ncell)) || (rc = dalloc(h, &h->geomx, size_t(GEOM_NF) * h->ncell)) ||
+  const size_t npad = h->march_plain ? 0 : size_t(B.nblk) * 2 * B.NNj * NNp;
+  if ((!h->march_plain && (rc = dalloc(h, &h->geom, size_t(GEOM_NF) * h->ncell))) ||
+      (rc = dalloc(h, &h->geomx, size_t(GEOM_NF) * h->ncell)) ||
       (rc = dalloc(h, &h->gmask, h->ncell)) ||
-      (rc = dalloc(h, &h->bcside, B.nblk)) || (rc = dalloc(h, &h->nodes_pad, size_t(B.nblk) * 2 * B.NNj * NNp)) ||
+      (rc = dalloc(h, &h->bcside, B.nblk)) || (npad && (rc = dalloc(h, &h->nodes_pad, npad))) ||
       (rc = dalloc(h, &degenerate, 1)))
     return rc;
   CK(cudaMemsetAsync(degenerate, 0, sizeof(int), h->stream));
-  CK(cudaMemsetAsync(h->nodes_pad, 0, sizeof(double) * size_t(B.nblk) * 2 * B.NNj * NNp, h->stream));
+  if (npad) CK(cudaMemsetAsync(h->nodes_pad, 0, sizeof(double) * npad, h->stream));
   // the exact build's geometry first: the fast one then writes the same mask,
   // side bits and padded nodes again, and both flag degenerate edges
   CK(exact::launch_geometry(B, h->geomx, h->gmask, h->bcside, degenerate, NNp, h->nodes_pad, h->stream));
-  CK(fast::launch_geometry(B, h->geom, h->gmask, h->bcside, degenerate, NNp, h->nodes_pad, h->stream));
+  if (!h->march_plain)
+    CK(fast::launch_geometry(B, h->geom, h->gmask, h->bcside, degenerate, NNp, h->nodes_pad, h->stream));
   int deg = 0;
   CK(cudaMemcpyAsync(&deg, degenerate, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (deg) return 0;
-  const uint32_t wi = mi + 4, nwi = mi + 6;
-  bool ok = encode3(&h->tmW[0], B.W, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4) &&
-            encode3(&h->tmW[1], B.W2, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4) &&
-            encode3(&h->tmG, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, wi, wj, G_K2 + 1) &&
-            encode3(&h->tmGx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, wi, wj, G_K2 + 1) &&
-            encode3(&h->tmN, h->nodes_pad, NNp, B.NNj, 2ull * B.nblk, nwi, wj, 2);
-  if (ok && h->W3) ok = encode3(&h->tmW[2], h->W3, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4);
-  if (!ok) return 0;
-  // update inputs of the explicit stages: boxes of the strip's columns x the
-  // most rows of a chunk
-  const uint32_t mj = fast::march_max_rows();
-  h->upd_ok = encode3(&h->tmU[0], B.U, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
-              encode3(&h->tmU[1], B.U2, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
-              encode3(&h->tmR, B.dUdt, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
-              encode3(&h->tmGA, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, 1) &&
-              encode3(&h->tmGF, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, GEOM_NF - G_RA) &&
-              encode3(&h->tmGAx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, 1) &&
-              encode3(&h->tmGFx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, GEOM_NF - G_RA);
+  if (!h->march_plain) {
+    const uint32_t wi = mi + 4, nwi = mi + 6;
+    bool ok = encode3(&h->tmW[0], B.W, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4) &&
+              encode3(&h->tmW[1], B.W2, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4) &&
+              encode3(&h->tmG, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, wi, wj, G_K2 + 1) &&
+              encode3(&h->tmGx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, wi, wj, G_K2 + 1) &&
+              encode3(&h->tmN, h->nodes_pad, NNp, B.NNj, 2ull * B.nblk, nwi, wj, 2);
+    if (ok && h->W3) ok = encode3(&h->tmW[2], h->W3, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4);
+    if (!ok) return 0;
+    // update inputs of the explicit stages: boxes of the strip's columns x the
+    // most rows of a chunk
+    const uint32_t mj = fast::march_max_rows();
+    h->upd_ok = encode3(&h->tmU[0], B.U, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
+                encode3(&h->tmU[1], B.U2, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
+                encode3(&h->tmR, B.dUdt, B.NCi, B.NCj, 4ull * B.nblk, mi, mj, 4) &&
+                encode3(&h->tmGA, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, 1) &&
+                encode3(&h->tmGF, h->geom, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, GEOM_NF - G_RA) &&
+                encode3(&h->tmGAx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, 1) &&
+                encode3(&h->tmGFx, h->geomx, B.NCi, B.NCj, uint64_t(GEOM_NF) * B.nblk, mi, mj, GEOM_NF - G_RA);
+  }
   const int per_sm =
       std::min(std::min(f32::march_ctas_per_sm(), fast::march_ctas_per_sm()), exact::march_ctas_per_sm());
   int sms = 0;
@@ -313,8 +322,14 @@ __global__ void uniform_state_kernel(Blocks B, long long ncell) {
   }
 }
 
+// The marching kernel's builds that take the handle's block width.
+bool march_applies(const e2d_handle* h, int prec) {
+  return h->march_ok && (!h->march_plain || prec == E2D_PREC_FP64_EXACT);
+}
+
 // Tunes one precision into sel_*[prec].
 int autotune_precision(e2d_handle* h, int prec) {
+  if (!march_applies(h, prec)) return 0;  // tiled, as initialised
   const TuneKey key{h->B.nci, h->B.ncj, h->B.nblk, prec, h->sc.flux};
   {
     std::lock_guard<std::mutex> lock(g_tune_mutex);
@@ -391,10 +406,13 @@ void apply_selection(e2d_handle* h) {
 int autotune_stage(e2d_handle* h) {
   if (!h->march_ok) return 0;
   // "tiled" / "march": one kernel without tuning (tests and comparisons of
-  // the two kernels; "march" with its default rows per chunk)
+  // the two kernels; "march" with its default rows per chunk, for even widths,
+  // "march_any" for odd ones too)
   const char* kind = getenv("CFFC_E2D_STAGE_KERNEL");
-  if (kind && (strcmp(kind, "tiled") == 0 || strcmp(kind, "march") == 0)) {
-    h->sel_march[0] = h->sel_march[1] = h->sel_march[2] = strcmp(kind, "march") == 0;
+  if (kind && (strcmp(kind, "tiled") == 0 || strcmp(kind, "march") == 0 || strcmp(kind, "march_any") == 0)) {
+    for (int p = 0; p < 3; ++p)
+      h->sel_march[p] = march_applies(h, p) && (strcmp(kind, "march_any") == 0 ||
+                                                (strcmp(kind, "march") == 0 && !h->march_plain));
     h->sel_rows[0] = h->sel_rows[1] = h->sel_rows[2] = fast::march_chunk_rows();
     apply_selection(h);
     return 0;

@@ -59,6 +59,7 @@ struct e2d_handle {
   int march_rows = 7;  // rows of a chunk
   double tune_us = 0.0;  // the autotuner's time of one explicit stage with the chosen kernel
   bool march_ok = false;  // geometry and tensor maps set up
+  bool march_plain = false;  // odd block width: no tensor maps, exact precision only
   // the autotuner's choice per precision (E2D_PREC_FP64, E2D_PREC_FP32,
   // E2D_PREC_FP64_EXACT)
   bool sel_march[3] = {false, false, false};

@@ -43,9 +43,15 @@
 // holds the quantities the reference computes from the grid alone, in its
 // order (e2d_march_args.h), and its results equal stage_kernel's bit for bit.
 //
-// Used when the block set allows it (even nci, no degenerate edges), for
-// every flux function (the Roe flux in an instance of its own);
-// stage_kernel covers the other block sets.
+// Used when the block set allows it (no degenerate edges), for every flux
+// function (the Roe flux in an instance of its own); stage_kernel covers the
+// other block sets.  Blocks an odd number of cells wide have no tensor maps
+// (rows off 16-byte boundaries): the exact build copies their windows by 8-byte
+// cp.async from all threads and reads the update inputs from global memory
+// (20 four-stage steps of 30 blocks of 37 x 29: 5.38 -> 3.91 ms against
+// stage_kernel, of 128 blocks of 45 x 45 22.8 -> 16.3 ms).  The fast builds do
+// not: stage_kernel is as fast there (1.89 against 2.00 ms, 8.16 against 7.89;
+// HLLC 2.63 against 2.55, 12.0 against 10.7).
 #pragma once
 #include "e2d_march_args.h"
 #include "e2d_pdl.cuh"
@@ -153,6 +159,10 @@ __device__ __forceinline__ void tma3(void* dst, const CUtensorMap* map, uint64_t
       "l"(reinterpret_cast<uint64_t>(map)), "r"(tc::smem_addr(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+// this thread's copies so far arrive on the barrier when they have landed
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_addr(bar)) : "memory");
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
@@ -171,6 +181,45 @@ __device__ __forceinline__ Chunk decode(const MarchArgs& m, long long g) {
   k.h = k.c == m.cps - 1 ? min(MJ, m.a.B.ncj - k.j0) : m.ch;
   k.r0 = (k.j0 + 1) % RR;
   return k;
+}
+
+#ifdef E2D_FAST
+constexpr bool PLAIN = false;  // windows without tensor copies
+#else
+constexpr bool PLAIN = true;
+#endif
+// A chunk's window without tensor copies, which want rows that start on 16-byte
+// boundaries: every thread copies, a warp a row at a time, zeros outside the
+// block.  The geometry and nodes, or the state (whose copies complete the
+// window: each thread's arrival on bar).
+__device__ __noinline__ void window_geo(const MarchArgs& m, Tile& T, const Chunk k) {
+  const Blocks& B = m.a.B;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int q = warp; q < (TG + 2) * WJ; q += NWARP) {
+    const int f = q / WJ, wj = q - f * WJ, J = k.j0 + wj;
+    const bool node = f >= TG;
+    const int rows = node ? B.NNj : B.NCj, cols = node ? B.NNi : B.NCi, width = node ? NWI : WI;
+    const double* base = node ? (f == TG ? B.X : B.Y) + size_t(k.b) * B.NNj * B.NNi
+                              : m.geom + (size_t(k.b) * GEOM_NF + f) * B.NCj * B.NCi;
+    double* dst = node ? &T.N[f - TG][wj][0] : &T.G[f][wj][0];
+    for (int c = lane; c < width; c += 32) {
+      const bool in = J < rows && k.i0 + c < cols;
+      tc::cp_async8(dst + c, in ? base + size_t(J) * cols + k.i0 + c : base, in);
+    }
+  }
+}
+__device__ __noinline__ void window_state(const MarchArgs& m, Tile& T, uint64_t* bar, const Chunk k) {
+  const Blocks& B = m.a.B;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int q = warp; q < 4 * WJ; q += NWARP) {
+    const int v = q / WJ, wj = q - v * WJ, J = k.j0 + wj;
+    const double* base = m.a.Win + (size_t(k.b) * 4 + v) * B.NCj * B.NCi;
+    for (int c = lane; c < WI; c += 32) {
+      const bool in = J < B.NCj && k.i0 + c < B.NCi;
+      tc::cp_async8(&T.W[v][wj][c], in ? base + size_t(J) * B.NCi + k.i0 + c : base, in);
+    }
+  }
+  cp_async_arrive(bar);
 }
 
 __device__ __forceinline__ PState<RT> wwin(const Tile& T, int wj, int wi) {
@@ -677,33 +726,38 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
   const long long g0 = m.nchunk * blockIdx.x / gridDim.x, g1 = m.nchunk * (blockIdx.x + 1) / gridDim.x;
   const size_t plane = size_t(B.NCi) * B.NCj;
 
-  // the window of chunk gg: the geometry and nodes, the state
+  // the window of chunk gg: the geometry and nodes, the state; by one thread,
+  // or by all without tensor copies
+  const bool plain_win = PLAIN && m.plain;
+  const bool issuer = plain_win || tid == 0;
   auto issue_geo = [&](const Chunk& k, int buf) {
+    if (plain_win) return window_geo(m, s.in[buf], k);
     uint64_t* bar = &s.full[buf];
     expect_tx(bar, TILE_BYTES);
     tma3(&s.in[buf].G[0][0][0], &m.tmG, bar, k.i0, k.j0, GEOM_NF * k.b);
     tma3(&s.in[buf].N[0][0][0], &m.tmN, bar, k.i0, k.j0, 2 * k.b);
   };
   auto issue_state = [&](const Chunk& k, int buf) {
+    if (plain_win) return window_state(m, s.in[buf], &s.full[buf], k);
     tma3(&s.in[buf].W[0][0][0], &m.tmW, &s.full[buf], k.i0, k.j0, 4 * k.b);
   };
   auto issue = [&](long long gg, int buf) {
     const Chunk k = decode(m, gg);
+    if (plain_win) issue_geo(k, buf);  // before the arrival that follows the state
     issue_state(k, buf);
-    issue_geo(k, buf);
+    if (!plain_win) issue_geo(k, buf);
   };
   // the first chunk's geometry before anything the stream computes (pdl_wait)
   if (tid == 0) {
-    tc::mbar_init(&s.full[0], 1);
-    tc::mbar_init(&s.full[1], 1);
+    tc::mbar_init(&s.full[0], plain_win ? THREADS : 1);
+    tc::mbar_init(&s.full[1], plain_win ? THREADS : 1);
     tc::mbar_init(&s.fullu, 1);
-    if (g0 < g1) issue_geo(decode(m, g0), 0);
   }
+  if (issuer && g0 < g1) issue_geo(decode(m, g0), 0);
   pdl_wait();
-  if (tid == 0) {
-    s.failed = *(volatile int*)B.status;
-    if (g0 < g1) issue_state(decode(m, g0), 0);
-  }
+  if (tid == 0) s.failed = *(volatile int*)B.status;
+  if (plain_win) __syncthreads();  // the barrier is set up before every thread's arrival
+  if (issuer && g0 < g1) issue_state(decode(m, g0), 0);
   __syncthreads();
   if (s.failed || g0 >= g1) {  // an earlier kernel failed: stop marching (uniform), the copies landed
     if (tid == 0 && g0 < g1) tc::mbar_wait(&s.full[0], 0u, WAIT_ITERS);
@@ -750,7 +804,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
     const int buf = NBUF == 2 ? (it & 1) : 0;
     const uint32_t par = NBUF == 2 ? (uint32_t(it >> 1) & 1u) : (uint32_t(it) & 1u);
     const Chunk k = decode(m, gg);
-    if (NBUF == 2 && tid == 0 && gg + 1 < g1) {
+    if (NBUF == 2 && issuer && gg + 1 < g1) {
       tc::fence_async_smem();  // the other buffer's generic reads come before its overwrite
       issue(gg + 1, buf ^ 1);
     }
@@ -784,6 +838,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
     if (__syncthreads_or(!ok)) {
       // a staging copy did not complete in time: record it, let the copies
       // in flight land (bounded), and stop
+      if (plain_win) tc::cp_async_wait();
       if (tid == 0) {
         set_status(B.status, ST_TIMEOUT, int(gg));
         tc::mbar_wait(&s.full[buf], par, WAIT_ITERS);
@@ -845,7 +900,7 @@ __global__ void __launch_bounds__(THREADS, MIN_CTAS) march_kernel(const __grid_c
       pcase = cs;
     }
     __syncthreads();
-    if (NBUF == 1 && tid == 0 && gg + 1 < g1) {
+    if (NBUF == 1 && issuer && gg + 1 < g1) {
       tc::fence_async_smem();  // this chunk's generic reads come before the overwrite
       issue(gg + 1, 0);
     }
@@ -1114,7 +1169,7 @@ cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, 
   if (e != cudaSuccess) return e;
   mk::bc_side_kernel<<<B.nblk, 32, 0, st>>>(B, bcside);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  mk::pad_nodes_kernel<<<1024, 256, 0, st>>>(B, NNp, nodes_pad);
+  if (nodes_pad) mk::pad_nodes_kernel<<<1024, 256, 0, st>>>(B, NNp, nodes_pad);
   return cudaGetLastError();
 }
 

@@ -45,6 +45,7 @@ struct MarchArgs {
   // RK stage 1 as [4 nblk][NCj][NCi], geometry plane G_RA alone and planes
   // G_RA .. G_VJY, as [GEOM_NF nblk][NCj][NCi]
   CUtensorMap tmU, tmR, tmGA, tmGF;
+  int plain;         // 1: rows of an odd number of cells, windows by cp.async (the exact build)
   int upd;           // 1: the update inputs of this launch arrive through these maps
   const double* geom;
   const unsigned char* mask;

@@ -143,6 +143,13 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   for (int q = 0; q < 32; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// Asynchronous 8-byte copy to shared memory, zero where !in.
+__device__ __forceinline__ void cp_async8(double* dst, const double* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(in ? 8 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Bulk copy of `bytes` (a multiple of 16, both addresses 16-byte aligned)
 // from global memory to this CTA's shared memory, completing on bar.
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
