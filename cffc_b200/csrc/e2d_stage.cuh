@@ -24,6 +24,7 @@
 #pragma once
 #include "e2d_device.cuh"
 #include "e2d_pdl.cuh"
+#include "e2d_tc.cuh"
 
 #ifndef E2D_NS
 #error "E2D_NS must name the kernel namespace"
@@ -289,12 +290,17 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   const int t = blockIdx.x % tiles;
   const int i0 = (t % a.tiles_i) * TI;   // interior index of the tile's first cell
   const int j0 = (t / a.tiles_i) * TJ;   // == array index of the halo origin
-  // the nodes before anything the stream computes (pdl_wait)
+  // ---- stage W and nodes (halo tile) --------------------------------------
+  // The nodes before anything the stream computes (pdl_wait); asynchronously, so
+  // that their latency, the state's and the flags' pass together (loaded one
+  // after the other, seven two-stage steps of 90 blocks of 27 x 25 took 666 us, so
+  // 644).
   for (int q = tid; q < NJ * NI; q += NTHREADS) {
     const int nj = q / NI, ni = q % NI, I = i0 + ni, J = j0 + nj;
     const bool in = I < B.NNi && J < B.NNj;
-    s.X[nj][ni] = in ? B.X[node_ix(B, b, J, I)] : 0.0;
-    s.Y[nj][ni] = in ? B.Y[node_ix(B, b, J, I)] : 0.0;
+    const size_t o = in ? node_ix(B, b, J, I) : 0;
+    tc::cp_async8(&s.X[nj][ni], B.X + o, in);
+    tc::cp_async8(&s.Y[nj][ni], B.Y + o, in);
   }
   pdl_wait();
   __shared__ int failed, frozen;
@@ -302,20 +308,23 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
     failed = *(volatile int*)B.status;
     frozen = B.freeze ? B.freeze[case_id(B, b)] : 0;
   }
-  __syncthreads();
-  if (failed) return;  // an earlier kernel failed: stop marching (uniform per CTA)
   const int cs = case_id(B, b);  // the block's case: its slot of the step history
-  if (B.case_active && !B.case_active[cs]) return;  // a finished case of a batch (uniform per CTA)
-  const double* dtmin_p = a.hist ? a.hist + 4 * ((*a.step) * B.ncase + cs) : nullptr;
-  const double g = B.g, gm1 = B.gm1, gm1i = B.gm1i;
-
-  // ---- stage W (halo tile) --------------------------------------
+  const bool running = !B.case_active || B.case_active[cs];
   for (int q = tid; q < 4 * HJ * HI; q += NTHREADS) {
     const int v = q / (HJ * HI), r = q % (HJ * HI), hj = r / HI, hi = r % HI;
     const int I = i0 + hi, J = j0 + hj;
-    s.W[v][hj][hi] = RT((I < B.NCi && J < B.NCj) ? a.Win[cell_var(B, b, v, J, I)] : 0.0);
+    const bool in = I < B.NCi && J < B.NCj;
+    if constexpr (sizeof(RT) == sizeof(double))
+      tc::cp_async8(reinterpret_cast<double*>(&s.W[v][hj][hi]), a.Win + (in ? cell_var(B, b, v, J, I) : 0), in);
+    else
+      s.W[v][hj][hi] = RT(in ? a.Win[cell_var(B, b, v, J, I)] : 0.0);
   }
+  tc::cp_async_wait();
   __syncthreads();
+  if (failed) return;  // an earlier kernel failed: stop marching (uniform per CTA)
+  if (!running) return;  // a finished case of a batch (uniform per CTA)
+  const double* dtmin_p = a.hist ? a.hist + 4 * ((*a.step) * B.ncase + cs) : nullptr;
+  const double g = B.g, gm1 = B.gm1, gm1i = B.gm1i;
 
   // ---- centroids of the halo tile ------------------------------------------
   for (int q = tid; q < HJ * HI; q += NTHREADS) {
