@@ -484,10 +484,10 @@ cudaError_t launch_explicit_stage(e2d_handle* h, int s, int fuse_next) {
 }
 
 // Ghost fill of the state stage s reads (s = 0: the solution (W, U)).
-cudaError_t ghost_fill_for(e2d_handle* h, int s) {
+cudaError_t ghost_fill_for(e2d_handle* h, int s, bool end_step) {
   Blocks B = h->B;
   if (s > 0) stage_buffers(h, stage_plan(h->sc, s).in, B.W, B.U);
-  return launch_ghost_fill(B, h->stream);
+  return launch_ghost_fill(B, h->stream, end_step ? h->hist : nullptr, h->step);
 }
 
 int ensure_recon(e2d_handle* h) {
@@ -613,19 +613,25 @@ cudaError_t launch_smoothed_stage(e2d_handle* h, int s) {
 // the last stage also reduces the next step's CFL minimum and residual
 // norms.  With residual smoothing the stages are split (residual,
 // smoothing, update) and every step starts with its own CFL and norms.
+// A step's end is part of the next step's first ghost fill (defer_step_end; the
+// run's last step is ended by e2d_rk_steps) unless a kernel before that fill
+// reads the step.
+bool defer_step_end(const e2d_handle* h) { return h->sc.rs_epsilon <= 0.0 && !h->freeze; }
+
 cudaError_t enqueue_step(e2d_handle* h) {
   cudaError_t e;
   const bool smooth = h->sc.rs_epsilon > 0.0;
   if (smooth && (e = enqueue_step_head(h))) return e;
   if ((e = launch_freeze_check(h))) return e;
   for (int stage = 1; stage <= h->sc.n_stage; ++stage) {
-    if ((e = ghost_fill_for(h, stage))) return e;
+    if ((e = ghost_fill_for(h, stage, stage == 1 && defer_step_end(h)))) return e;
     if (smooth) {
       if ((e = launch_smoothed_stage(h, stage))) return e;
     } else if ((e = launch_explicit_stage(h, stage, stage == h->sc.n_stage))) {
       return e;
     }
   }
+  if (defer_step_end(h)) return cudaSuccess;
   return launch_step_end(h->hist, h->step, smooth ? 0 : 1, h->B.ncase, smooth ? 0 : 1, h->stream);
 }
 
@@ -818,13 +824,13 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
       (rc = dalloc(h, &B.W2, 4 * h->ncell)) || (rc = dalloc(h, &B.U2, 4 * h->ncell)) ||
       (rc = dalloc(h, &B.dUdt, 4 * h->ncell)) ||
       (rc = dalloc(h, &B.dt, h->ncell)) || (rc = dalloc(h, &B.status, 2)) ||
-      (rc = dalloc(h, &h->step, 1)) || (rc = dalloc(h, &h->part, size_t(3) * B.nblk)))
+      (rc = dalloc(h, &h->step, 2)) || (rc = dalloc(h, &h->part, size_t(3) * B.nblk)))
     return fail(rc, h);
   if (cudaMemset(B.W, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(B.U, 0, sizeof(double) * 4 * h->ncell) ||
       cudaMemset(B.W2, 0, sizeof(double) * 4 * h->ncell) ||
       cudaMemset(B.U2, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(B.dUdt, 0, sizeof(double) * 4 * h->ncell) ||
       cudaMemset(B.dt, 0, sizeof(double) * h->ncell) || cudaMemset(B.status, 0, sizeof(int) * 2) ||
-      cudaMemset(h->step, 0, sizeof(int)))
+      cudaMemset(h->step, 0, 2 * sizeof(int)))
     return fail(E2D_ERR_CUDA, h);
   unsigned char* flags = nullptr;
   double2* nrm = nullptr;
@@ -1131,7 +1137,7 @@ int e2d_rk_steps(e2d_handle* h, int n_steps, double* hist) {
   // the stage kernels do not write the optional reconstruction arrays
   const Blocks saved = h->B;
   h->B.dWdx = h->B.dWdy = h->B.phi = nullptr;
-  CK(cudaMemsetAsync(h->step, 0, sizeof(int), h->stream));
+  CK(cudaMemsetAsync(h->step, 0, 2 * sizeof(int), h->stream));
   CK(enqueue_step_head(h));
   // one graph of a step and, for long runs, one of STEP_GROUP steps
   for (int k = 0; k < 2; ++k) {
@@ -1156,6 +1162,7 @@ int e2d_rk_steps(e2d_handle* h, int n_steps, double* hist) {
   if (h->step_graph[1] && n_steps >= STEP_GROUP_MIN)
     for (; s + STEP_GROUP <= n_steps; s += STEP_GROUP) CK(cudaGraphLaunch(h->step_graph[1], h->stream));
   for (; s < n_steps; ++s) CK(cudaGraphLaunch(h->step_graph[0], h->stream));
+  if (defer_step_end(h)) CK(launch_step_end(h->hist, h->step, 1, h->B.ncase, 1, h->stream));
   if (h->sc.n_stage >= 2) {
     // The reference keeps one state array, so after a multistage step its
     // ghost cells hold the last stage's exchange and BCs; here those went

@@ -22,7 +22,7 @@ struct e2d_handle {
   std::vector<void*> allocs;
   double* hist = nullptr;  // [hist_cap][4]
   int hist_cap = 0;
-  int* step = nullptr;     // device step counter
+  int* step = nullptr;     // device step counter; whether the step before is to be ended
   double* part = nullptr;  // [nblk][3] norm partials
   bool recon_out = false;  // dWdx/dWdy/phi arrays allocated
   // third stage state (schemes of three or more stages) and the second and
@@ -101,7 +101,7 @@ cudaError_t launch_stage_any(e2d_handle* h, int mode, int fuse_next);
 cudaError_t launch_stage_args(e2d_handle* h, e2d::StageArgs& a);
 // Newton-Krylov over the sub-batches of a mixed-shape batch (e2d_nks).
 int composite_nks(e2d_handle* h, const e2d_nks_params* p, e2d_nks_step* hist, int* n_steps);
-cudaError_t ghost_fill_for(e2d_handle* h, int mode);
+cudaError_t ghost_fill_for(e2d_handle* h, int mode, bool end_step = false);
 int ensure_hist(e2d_handle* h, int n);
 void nks_free(e2d_handle* h);
 void nks_drop_graphs(e2d_handle* h);

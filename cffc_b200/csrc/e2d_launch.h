@@ -53,7 +53,8 @@ inline void stage_tile(int precision, int* ti, int* tj) {
   else if (precision == E2D_PREC_FP32) { *ti = f32::tile_i(); *tj = f32::tile_j(); }
   else { *ti = fast::tile_i(); *tj = fast::tile_j(); }
 }
-cudaError_t launch_ghost_fill(const Blocks& B, cudaStream_t st);
+// with hist (step [2]: the step, one to end): the step before is ended as well
+cudaError_t launch_ghost_fill(const Blocks& B, cudaStream_t st, double* hist = nullptr, int* step = nullptr);
 cudaError_t launch_edge_setup(const Blocks& B, unsigned char* flags, double2* nrm, cudaStream_t st);
 cudaError_t launch_cfl(const Blocks& B, double* hist, const int* step, cudaStream_t st);
 cudaError_t launch_norms(const Blocks& B, double* part, double* hist, const int* step, cudaStream_t st);
