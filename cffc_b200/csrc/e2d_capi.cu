@@ -143,9 +143,12 @@ void stage_buffers(e2d_handle* h, int k, double*& W, double*& U) {
 
 // The stage kernel for a stage: the column-marching kernel where the handle
 // allows it (no degenerate edges; odd widths in exact precision only) and the
-// autotuner chose it, else the tiled stage kernel.
+// autotuner chose it, else the tiled stage kernel.  Residuals and Frechet
+// products of the fast precisions, whose two kernels round differently, take
+// the marching kernel wherever it applies: Newton-Krylov runs then do not depend
+// on the block count's tuning (a batch's case equals its solo run).
 cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
-  if (h->march) {
+  if (a.mode == 0 || a.mode == 3 ? h->march_lin : h->march) {
     const bool ex = h->sc.precision == E2D_PREC_FP64_EXACT;
     const CUtensorMap* tw = nullptr;
     if (a.Win == h->B.W) tw = &h->tmW[0];
@@ -358,7 +361,8 @@ int autotune_precision(e2d_handle* h, int prec) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
-  TuneChoice best{true, h->march_rows, 1e30f};
+  TuneChoice best{true, h->march_rows, 1e30f};  // rows: the best marching candidate's
+  float march_us = 1e30f;
   for (int cand = 0; cand <= 5; ++cand) {  // 0: tiled; 1..5: marching, 4..8 rows
     h->march = cand > 0;
     h->march_rows = cand > 0 ? 3 + cand : h->march_rows;
@@ -375,7 +379,14 @@ int autotune_precision(e2d_handle* h, int prec) {
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     const float us = 1000.f * ms / 3.f;
-    if (us < best.us) best = TuneChoice{h->march, h->march_rows, us};
+    if (us < best.us) {
+      best.us = us;
+      best.march = h->march;
+    }
+    if (h->march && us < march_us) {
+      march_us = us;
+      best.rows = h->march_rows;
+    }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -392,10 +403,11 @@ int autotune_precision(e2d_handle* h, int prec) {
 void apply_selection(e2d_handle* h) {
   const int p = h->sc.precision;
   if (!h->march_ok) {
-    h->march = false;
+    h->march = h->march_lin = false;
     return;
   }
   h->march = h->sel_march[p];
+  h->march_lin = h->sel_lin[p];
   h->march_rows = h->sel_rows[p];
   h->tune_us = h->sel_us[p];
 }
@@ -413,6 +425,7 @@ int autotune_stage(e2d_handle* h) {
     for (int p = 0; p < 3; ++p)
       h->sel_march[p] = march_applies(h, p) && (strcmp(kind, "march_any") == 0 ||
                                                 (strcmp(kind, "march") == 0 && !h->march_plain));
+    for (int p = 0; p < 3; ++p) h->sel_lin[p] = h->sel_march[p];
     h->sel_rows[0] = h->sel_rows[1] = h->sel_rows[2] = fast::march_chunk_rows();
     apply_selection(h);
     return 0;
@@ -428,6 +441,8 @@ int autotune_stage(e2d_handle* h) {
   if ((rc = autotune_precision(h, E2D_PREC_FP64)) || (rc = autotune_precision(h, E2D_PREC_FP32)) ||
       (rc = autotune_precision(h, E2D_PREC_FP64_EXACT)))
     return rc;
+  for (int p = 0; p < 3; ++p)
+    h->sel_lin[p] = p == E2D_PREC_FP64_EXACT ? h->sel_march[p] : march_applies(h, p);
   apply_selection(h);
   // the handle starts from a clean slate
   const size_t nb = sizeof(double) * 4 * h->ncell;

@@ -63,6 +63,8 @@ struct e2d_handle {
   // the autotuner's choice per precision (E2D_PREC_FP64, E2D_PREC_FP32,
   // E2D_PREC_FP64_EXACT)
   bool sel_march[3] = {false, false, false};
+  // the marching kernel for residuals and Frechet products (the current precision's; all)
+  bool march_lin = false, sel_lin[3] = {false, false, false};
   int sel_rows[3] = {7, 7, 7};
   double sel_us[3] = {0.0, 0.0, 0.0};
   // captured explicit steps: one, STEP_GROUP of them

@@ -48,10 +48,11 @@
 // other block sets.  Blocks an odd number of cells wide have no tensor maps
 // (rows off 16-byte boundaries): the exact build copies their windows by 8-byte
 // cp.async from all threads and reads the update inputs from global memory
-// (20 four-stage steps of 30 blocks of 37 x 29: 5.38 -> 3.91 ms against
-// stage_kernel, of 128 blocks of 45 x 45 22.8 -> 16.3 ms).  The fast builds do
-// not: stage_kernel is as fast there (1.89 against 2.00 ms, 8.16 against 7.89;
-// HLLC 2.63 against 2.55, 12.0 against 10.7).
+// (20 four-stage steps of 30 blocks of 63 x 63: 6.24 ms against stage_kernel's
+// 8.64; of 37 x 29, two short tiles there, 3.91 against 3.57: the autotuner
+// times both).  The fast builds do not: stage_kernel is faster there (30 blocks
+// of 37 x 29 1.52 against 1.89 ms, HLLC 1.98 against 2.63; 128 blocks of 45 x 45
+// 5.95 against 8.16).
 #pragma once
 #include "e2d_march_args.h"
 #include "e2d_pdl.cuh"

@@ -77,6 +77,16 @@ constexpr int RI = TI + 2, RJ = TJ + 2; // cells reconstructed (tile + 1 ring)
 constexpr int NTHREADS = E2D_THREADS;
 static_assert(NTHREADS >= TI * TJ && NTHREADS % 32 == 0, "one thread per tile cell at least");
 
+// q / d and q % d of a work item's rows of d items, d >= 1: one multiplication,
+// exact for q * d < 65536 (at most 4 x 12 x 36 items in rows of at most 37).
+struct Rows {
+  unsigned d, m;
+  __device__ __forceinline__ explicit Rows(int d_) : d(d_), m(65536u / unsigned(d_) + 1u) {}
+  __device__ __forceinline__ int row(int q) const { return int((unsigned(q) * m) >> 16); }
+  __device__ __forceinline__ int col(int q, int row) const { return q - row * int(d); }
+};
+static_assert(4 * HJ * HI * NI < 65536 && (TI + 1) * TJ * (TI + 1) < 65536, "Rows is exact");
+
 struct Smem {
   RT W[4][HJ][HI];
   double X[NJ][NI], Y[NJ][NI];
@@ -288,19 +298,26 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   const int tiles = a.tiles_i * a.tiles_j;
   const int b = blockIdx.x / tiles;
   const int t = blockIdx.x % tiles;
-  const int i0 = (t % a.tiles_i) * TI;   // interior index of the tile's first cell
-  const int j0 = (t / a.tiles_i) * TJ;   // == array index of the halo origin
+  // The block's cells in tiles of equal extent, at most TI x TJ, and the work
+  // items of the tile's own extent: a block of 37 columns is two tiles of 19
+  // and 18 whose reconstructions and faces take one and two rounds of the CTA,
+  // not of 32 and 5 with two and two (20 four-stage steps of 30 such blocks of 29
+  // rows 2.46 -> 1.98 ms, of 128 blocks of 45 x 45 7.89 -> 5.95 ms).
+  const int tw = (B.nci + a.tiles_i - 1) / a.tiles_i, th = (B.ncj + a.tiles_j - 1) / a.tiles_j;
+  const int i0 = (t % a.tiles_i) * tw;   // interior index of the tile's first cell
+  const int j0 = (t / a.tiles_i) * th;   // == array index of the halo origin
+  const int nci_t = min(tw, B.nci - i0), ncj_t = min(th, B.ncj - j0);
   // ---- stage W and nodes (halo tile) --------------------------------------
   // The nodes before anything the stream computes (pdl_wait); asynchronously, so
   // that their latency, the state's and the flags' pass together (loaded one
   // after the other, seven two-stage steps of 90 blocks of 27 x 25 took 666 us, so
   // 644).
-  for (int q = tid; q < NJ * NI; q += NTHREADS) {
-    const int nj = q / NI, ni = q % NI, I = i0 + ni, J = j0 + nj;
-    const bool in = I < B.NNi && J < B.NNj;
-    const size_t o = in ? node_ix(B, b, J, I) : 0;
-    tc::cp_async8(&s.X[nj][ni], B.X + o, in);
-    tc::cp_async8(&s.Y[nj][ni], B.Y + o, in);
+  const Rows rn(nci_t + 5), rh(nci_t + 4);
+  for (int q = tid; q < (ncj_t + 5) * (nci_t + 5); q += NTHREADS) {
+    const int nj = rn.row(q), ni = rn.col(q, nj);
+    const size_t o = node_ix(B, b, j0 + nj, i0 + ni);
+    tc::cp_async8(&s.X[nj][ni], B.X + o, true);
+    tc::cp_async8(&s.Y[nj][ni], B.Y + o, true);
   }
   pdl_wait();
   __shared__ int failed, frozen;
@@ -310,14 +327,15 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   }
   const int cs = case_id(B, b);  // the block's case: its slot of the step history
   const bool running = !B.case_active || B.case_active[cs];
-  for (int q = tid; q < 4 * HJ * HI; q += NTHREADS) {
-    const int v = q / (HJ * HI), r = q % (HJ * HI), hj = r / HI, hi = r % HI;
-    const int I = i0 + hi, J = j0 + hj;
-    const bool in = I < B.NCi && J < B.NCj;
+  const int hrows = ncj_t + 4;
+  for (int q = tid; q < 4 * hrows * (nci_t + 4); q += NTHREADS) {
+    const int r = rh.row(q), hi = rh.col(q, r);
+    const int v = (r >= hrows) + (r >= 2 * hrows) + (r >= 3 * hrows), hj = r - v * hrows;
+    const double* w = a.Win + cell_var(B, b, v, j0 + hj, i0 + hi);
     if constexpr (sizeof(RT) == sizeof(double))
-      tc::cp_async8(reinterpret_cast<double*>(&s.W[v][hj][hi]), a.Win + (in ? cell_var(B, b, v, J, I) : 0), in);
+      tc::cp_async8(reinterpret_cast<double*>(&s.W[v][hj][hi]), w, true);
     else
-      s.W[v][hj][hi] = RT(in ? a.Win[cell_var(B, b, v, J, I)] : 0.0);
+      s.W[v][hj][hi] = RT(*w);
   }
   tc::cp_async_wait();
   __syncthreads();
@@ -327,8 +345,8 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   const double g = B.g, gm1 = B.gm1, gm1i = B.gm1i;
 
   // ---- centroids of the halo tile ------------------------------------------
-  for (int q = tid; q < HJ * HI; q += NTHREADS) {
-    const int hj = q / HI, hi = q % HI;
+  for (int q = tid; q < hrows * (nci_t + 4); q += NTHREADS) {
+    const int hj = rh.row(q), hi = rh.col(q, hj);
     double xc, yc, area;
     E2D_QC(s.X[hj][hi], s.Y[hj][hi], s.X[hj][hi + 1], s.Y[hj][hi + 1], s.X[hj + 1][hi + 1],
                   s.Y[hj + 1][hi + 1], s.X[hj + 1][hi], s.Y[hj + 1][hi], xc, yc, area);
@@ -338,12 +356,11 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
   __syncthreads();
 
   // ---- least-squares gradients and limiter of the ring-1 region -----------
-  const int nci_t = min(TI, B.nci - i0), ncj_t = min(TJ, B.ncj - j0);
-  for (int q = tid; q < RJ * RI; q += NTHREADS) {
-    const int rj = q / RI, ri = q % RI;
+  const Rows rr(nci_t + 2);
+  for (int q = tid; q < (ncj_t + 2) * (nci_t + 2); q += NTHREADS) {
+    const int rj = rr.row(q), ri = rr.col(q, rj);
     const int hi = ri + 1, hj = rj + 1;
     const int I = i0 + hi, J = j0 + hj;
-    if (ri > nci_t + 1 || rj > ncj_t + 1) continue;
     int di[8], dj[8];
     const int n = lsq_stencil(B, b, I, J, di, dj);
     if (n == 0) {
@@ -426,15 +443,15 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
 
   // ---- face fluxes -----------------------------------------------------------
   const int ICl = NG, ICu = B.nci + NG - 1, JCl = NG, JCu = B.ncj + NG - 1;
-  const int nfi = (TI + 1) * TJ, nfj = TI * (TJ + 1);
+  const int nfi = (nci_t + 1) * ncj_t, nfj = nci_t * (ncj_t + 1);
+  const Rows ri_f(nci_t + 1), rj_f(nci_t);
   for (int q = tid; q < nfi + nfj; q += NTHREADS) {
     PState<RT> wl, wr;
     double nx, ny, l;
     int fi, fj;
     bool is_i = q < nfi;
     if (is_i) {
-      fj = q / (TI + 1); fi = q % (TI + 1);
-      if (fi > nci_t || fj >= ncj_t) continue;
+      fj = ri_f.row(q); fi = ri_f.col(q, fj);
       // face between halo cells (fi+1, fj+2) and (fi+2, fj+2): east face of the left cell
       const int hl = fi + 1, hj = fj + 2, I = i0 + hl, J = j0 + hj;
       const double ax = s.X[hj + 1][hl + 1], ay = s.Y[hj + 1][hl + 1];  // node (I+1, J+1)
@@ -460,8 +477,7 @@ __global__ void __launch_bounds__(NTHREADS, E2D_MIN_CTAS) stage_kernel(StageArgs
       }
     } else {
       const int q2 = q - nfi;
-      fj = q2 / TI; fi = q2 % TI;
-      if (fi >= nci_t || fj > ncj_t) continue;
+      fj = rj_f.row(q2); fi = rj_f.col(q2, fj);
       // face between halo cells (fi+2, fj+1) and (fi+2, fj+2): north face of the lower cell
       const int hi = fi + 2, hl = fj + 1, I = i0 + hi, J = j0 + hl;
       const double ax = s.X[hl + 1][hi], ay = s.Y[hl + 1][hi];          // node (I, J+1)
