@@ -811,9 +811,9 @@ def main():
 
     line = None
     if rank == 0:
-        # per time step: slot init, (ghost fill + stage) per stage, step end;
-        # per e2d_rk_steps call: slot init, CFL, two norm kernels
-        launches_per_rk = 2 + 2 * bs.scheme.n_stage
+        # per time step: a ghost fill and a stage kernel per stage; per run two slot resets, CFL,
+        # two norm kernels, the last step's end and the ghost copy
+        launches_per_rk = 2 * bs.scheme.n_stage
         line = {
             "metric": "Mcell-updates/s (Roe+limiter residual, explicit RK2)",
             "value": round(value, 3), "unit": "Mcell-updates/s", "n_gpus": world,
@@ -834,7 +834,7 @@ def main():
             "path_roofline": {"bytes_per_cell_update": 240,
                               "achieved_gbs": round(240 * cell_updates / (ms * 1e-3) / 1e9, 2),
                               "frac": round(240 * cell_updates / (ms * 1e-3) / 1e9 / hbm, 4)},
-            "gpu_launches": args.steps * (args.rk_steps * launches_per_rk + 4),
+            "gpu_launches": args.steps * (args.rk_steps * launches_per_rk + 7),
             "clocks": clk.summary(),
         }
         if args.precision == "fp32":
