@@ -125,7 +125,9 @@ struct Team {
   // adds each slot's warp sums in order.  A cluster's CTA adds its slots into
   // the two lanes' sums and sends their sum to every CTA; a grid team's CTA
   // sends its slots to global memory, its threads wait for a slot each and
-  // every warp adds all of them.
+  // every warp adds all of them.  Every CTA of a team sends something and waits
+  // for all the others in every round: the sums alternate between two buffers,
+  // and a CTA that nobody waited for could find its round's overwritten.
   __device__ double total(int count, int nl, int base) {
     const int lane = threadIdx.x & 31;
     __syncthreads();
@@ -159,7 +161,9 @@ struct Team {
     ++tag;
     if (threadIdx.x < 32)
       for (int q = lane; q < nl; q += 32) st_tagged(gp + base + q, slot_sum(q), tag);
-    for (int q = threadIdx.x; q < count; q += AT) {
+    // the CTAs without a slot (rank - base of them below this one) post an empty one after the slots
+    if (threadIdx.x == 0 && nl == 0) st_tagged(gp + count + rank - base, 0.0, tag);
+    for (int q = threadIdx.x; q < max(count, size); q += AT) {
       double v;
       for (uint32_t it = 0; ld_tagged(gp + q, v) != tag;) {
         if (!ok || ++it >= A_WAIT) {
