@@ -128,7 +128,11 @@ struct Team {
   // every warp adds all of them.  Every CTA of a team sends something and waits
   // for all the others in every round: the sums alternate between two buffers,
   // and a CTA that nobody waited for could find its round's overwritten.
-  __device__ double total(int count, int nl, int base) {
+  // With `fence` the team's earlier writes to global memory are visible to every
+  // thread afterwards: the CTA barrier and the sender's fence take the CTA's
+  // writes along with the sum, the receivers' fences order them before the
+  // threads behind the closing CTA barrier.
+  __device__ double total(int count, int nl, int base, bool fence = false) {
     const int lane = threadIdx.x & 31;
     __syncthreads();
     if (CLUSTER) {
@@ -159,6 +163,7 @@ struct Team {
     ulonglong2* gp = part + size_t(round & 1) * slots;
     double* sp = copy + size_t(round & 1) * slots;
     ++tag;
+    if (fence && threadIdx.x < 32) __threadfence();
     if (threadIdx.x < 32)
       for (int q = lane; q < nl; q += 32) st_tagged(gp + base + q, slot_sum(q), tag);
     // the CTAs without a slot (rank - base of them below this one) post an empty one after the slots
@@ -174,6 +179,7 @@ struct Team {
       }
       sp[q] = v;
     }
+    if (fence) __threadfence();
     ok = __syncthreads_and(ok) != 0;
     ++round;
     double t = 0.0;
@@ -189,13 +195,11 @@ struct Team {
   }
   // every thread: the team's writes to global memory are visible to the team
   __device__ void barrier() {
-    __threadfence();
     if (CLUSTER) {
-      tc::cluster_sync();
+      tc::cluster_sync();  // (a release and an acquire)
     } else {
       if (threadIdx.x < VT / 32) red[0][threadIdx.x] = 0.0;
-      total(size, 1, rank);  // a round of one empty slot per CTA
-      __threadfence();
+      total(size, 1, rank, true);  // a round of one empty slot per CTA
     }
   }
 };
