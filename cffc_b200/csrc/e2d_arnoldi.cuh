@@ -118,7 +118,7 @@ struct Team {
   double* copy;            // grid: the same in shared memory
   int slots;
   unsigned long long tag;  // grid: rounds of all launches so far
-  bool ok;           // no wait has run out (once one has, none is waited for)
+  bool ok;           // no wait has run out (once one has, the CTA sends and waits no more)
 
   // every thread: the team's sum of `count` slots, of which this CTA holds nl
   // (slot base + step * i with its warp sums in red[i]).  The CTA's first warp
@@ -149,7 +149,7 @@ struct Team {
         uint64_t* bar = &s.bar[round & 1];
         t += __shfl_xor_sync(0xffffffffu, t, 1);
         if (lane == 0) tc::mbar_expect_tx(bar, ATEAM * 8u);
-        if (lane < ATEAM)
+        if (ok && lane < ATEAM)
           st_async(tc::peer_addr(tc::smem_addr(&s.part[round & 1][base]), lane), t,
                    tc::peer_addr(tc::smem_addr(bar), lane));
         if (ok) ok = tc::mbar_wait_warp(bar, uint32_t(round >> 1) & 1u, A_WAIT);
@@ -164,10 +164,10 @@ struct Team {
     double* sp = copy + size_t(round & 1) * slots;
     ++tag;
     if (fence && threadIdx.x < 32) __threadfence();
-    if (threadIdx.x < 32)
+    if (ok && threadIdx.x < 32)
       for (int q = lane; q < nl; q += 32) st_tagged(gp + base + q, slot_sum(q), tag);
     // the CTAs without a slot (rank - base of them below this one) post an empty one after the slots
-    if (threadIdx.x == 0 && nl == 0) st_tagged(gp + count + rank - base, 0.0, tag);
+    if (ok && threadIdx.x == 0 && nl == 0) st_tagged(gp + count + rank - base, 0.0, tag);
     for (int q = threadIdx.x; q < max(count, size); q += AT) {
       double v;
       for (uint32_t it = 0; ld_tagged(gp + q, v) != tag;) {
@@ -444,7 +444,10 @@ __global__ void __launch_bounds__(AT, 1) arnoldi_kernel(const __grid_constant__ 
       if (f) a.active[c] = 0;
       team_progress(a, f ? 0 : 1);
     }
-    if (f) {  // uniform over the team
+    if (f) {  // uniform over the team's CTAs whose waits have not run out
+      // one whose wait has stays until the others, which may go on to the next
+      // step's head, have sent to it for the last time
+      if (CLUSTER && !team.ok && a.next == NEXT_JACOBI) tc::cluster_sync();  // their barrier()
       team_exit(team, a.ground + c);
       return;
     }

@@ -762,7 +762,7 @@ struct e2d_nks_state {
   unsigned* counter = nullptr; // [ncase] arrivals of the reduction CTAs
   int team = 0;              // arnoldi_kernel: 1 a cluster per case, 2 a share of the GPU per case, 0 separate kernels
   int team_ctas = 0, team_ctaslots = 0, team_slots = 0;
-  size_t team_smem = 0;
+  size_t team_smem = 0, team_sums = 0;
   int* team_cnt = nullptr;   // [2]
   int* team_cta0 = nullptr;                   // [ncase + 1]
   ulonglong2* team_part = nullptr;
@@ -853,6 +853,16 @@ size_t team_work(const e2d_handle* h, int nb, int size) {
   return std::max(size_t((ns + size - 1) / size) * len, size_t((nsc + size - 1) / size) * lenc * 2) * sizeof(double2);
 }
 
+// No round of a reduction has run: when set up, and after a failed solve, whose
+// teams may have left sums of rounds that the next one's would take for theirs.
+int team_clear(e2d_handle* h) {
+  e2d_nks_state* s = h->nks;
+  E2D_CK(cudaMemsetAsync(s->team_cnt, 0, 2 * sizeof(int), h->stream));
+  E2D_CK(cudaMemsetAsync(s->team_round, 0, sizeof(unsigned long long) * s->ncase, h->stream));
+  E2D_CK(cudaMemsetAsync(s->team_part, 0, sizeof(ulonglong2) * s->team_sums, h->stream));
+  return 0;
+}
+
 // How the Arnoldi steps of this handle run: a cluster of 16 CTAs per case
 // where every case's vector fits the clusters' registers (64 slots of 512
 // entries, 12 blocks of 32 x 32; a quarter more in shared memory still wins)
@@ -884,13 +894,11 @@ int team_setup(e2d_handle* h) {
   int nbmax = 0;
   for (int c = 0; c < C; ++c) nbmax = std::max(nbmax, start[c + 1] - start[c]);
   s->team = 0;
+  s->team_sums = 2 * (size_t(B.nblk) * maxch + sms);
   if ((rc = nalloc(s, &s->team_cnt, 2)) || (rc = nalloc(s, &s->team_round, C)) ||
       (rc = nalloc(s, &s->team_cta0, C + 1)) ||
-      (rc = nalloc(s, &s->team_part, 2 * (size_t(B.nblk) * maxch + sms))))
+      (rc = nalloc(s, &s->team_part, s->team_sums)) || (rc = team_clear(h)))
     return rc;
-  E2D_CK(cudaMemsetAsync(s->team_cnt, 0, 2 * sizeof(int), h->stream));
-  E2D_CK(cudaMemsetAsync(s->team_round, 0, sizeof(unsigned long long) * C, h->stream));
-  E2D_CK(cudaMemsetAsync(s->team_part, 0, sizeof(ulonglong2) * 2 * (size_t(B.nblk) * maxch + sms), h->stream));
   // the Arnoldi kernel's shared memory with `slots` slots a CTA
   auto smem = [&](int slots, int all, size_t work) { return arnoldi_head(slots, all, s->m) + work; };
   auto slots_of = [&](int nb, int size) { return (nb * maxch + size - 1) / size; };
@@ -1500,7 +1508,10 @@ int gmres(e2d_handle* h, const e2d_nks_params& p, const std::vector<double>& tol
     E2D_CK(cudaMemcpyAsync(hi + C, D.flags, sizeof(int) * C, cudaMemcpyDeviceToHost, h->stream));
     E2D_CK(cudaMemcpyAsync(hi + 2 * C, D.err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     E2D_CK(cudaStreamSynchronize(h->stream));
-    if (hi[2 * C]) return hi[2 * C];
+    if (hi[2 * C]) {
+      if ((rc = team_clear(h))) return rc;
+      return hi[2 * C];
+    }
     bool more = false;
     for (int c = 0; c < C; ++c) {
       if (!on[c]) continue;
