@@ -142,11 +142,10 @@ void stage_buffers(e2d_handle* h, int k, double*& W, double*& U) {
 }
 
 // The stage kernel for a stage: the column-marching kernel where the handle
-// allows it (no degenerate edges; odd widths in exact precision only) and the
-// autotuner chose it, else the tiled stage kernel.  Residuals and Frechet
-// products of the fast precisions, whose two kernels round differently, take
-// the marching kernel wherever it applies: Newton-Krylov runs then do not depend
-// on the block count's tuning (a batch's case equals its solo run).
+// allows it (no degenerate edges; odd widths in exact precision only) and it is
+// the one for the block width (autotune_precision), else the tiled stage kernel.
+// Residuals and Frechet products of the fast precisions take the marching
+// kernel wherever it applies.
 cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
   if (a.mode == 0 || a.mode == 3 ? h->march_lin : h->march) {
     const bool ex = h->sc.precision == E2D_PREC_FP64_EXACT;
@@ -296,7 +295,8 @@ int setup_march(e2d_handle* h) {
 // The candidates -- the tiled kernel and the marching kernel with 4 to 8
 // rows per chunk -- are timed on the handle's own block set (a uniform
 // state, an explicit stage 1 per launch, one warm-up and three timed
-// launches each) when the handle is created; the fastest is kept.  Choices
+// launches each) when the handle is created; the fastest is kept, among those
+// of the kernel that prefers_march names in the fast precisions.  Choices
 // are cached per (block shape, block count, precision, flux function) for
 // the process.
 struct TuneKey {
@@ -330,6 +330,24 @@ bool march_applies(const e2d_handle* h, int prec) {
   return h->march_ok && (!h->march_plain || prec == E2D_PREC_FP64_EXACT);
 }
 
+// The fast precisions' two kernels round differently, so which one runs a block
+// set's explicit stages depends on the block width, the precision and the flux
+// alone, not on the number of blocks or a clock: a case gives the same bits in a
+// batch as alone, and in every process.  (The rows of a chunk change no cell's
+// bits, nor does the kernel in exact precision: there the clock decides.)
+// The marching kernel works in strips of 32 columns whose last one costs nearly
+// a full one's time, the tiled kernel in tiles of equal width.  Its time over
+// the tiled kernel's, mean of 4 to 256 blocks of 8 to 64 rows (B200): FP64 Roe 1.08 at
+// 8 columns, 1.05 at 14, 1.01 at 18, 0.94 at 20, 0.79 at 32, 0.99 at 34 and 36,
+// 0.95 at 40, 0.76 at 64; the other fluxes (HLLE, HLLC, AUSM+) 1.20, 1.35, 1.12 at 8,
+// 1.12, 1.23, 1.05 at 18, 1.02, 1.09, 0.98 at 20, 1.13, 1.25, 1.05 at 36, 1.04, 1.10,
+// 1.00 at 38; FP32 1.07 to 1.15 at 8, 1.01 to 1.08 at 14, 0.98 to 1.04 at 16, at most
+// 1.04 at 34 and 36.  Either kernel wins by up to 30 % at some counts of blocks.
+bool prefers_march(int nci, int prec, int flux) {
+  if (prec == E2D_PREC_FP32) return nci > 14;
+  return nci > 18 && (flux == E2D_FLUX_ROE || nci <= 32 || nci > 36);
+}
+
 // Tunes one precision into sel_*[prec].
 int autotune_precision(e2d_handle* h, int prec) {
   if (!march_applies(h, prec)) return 0;  // tiled, as initialised
@@ -361,9 +379,10 @@ int autotune_precision(e2d_handle* h, int prec) {
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
+  const bool fixed = prec != E2D_PREC_FP64_EXACT, fixed_march = fixed && prefers_march(h->B.nci, prec, h->sc.flux);
   TuneChoice best{true, h->march_rows, 1e30f};  // rows: the best marching candidate's
   float march_us = 1e30f;
-  for (int cand = 0; cand <= 5; ++cand) {  // 0: tiled; 1..5: marching, 4..8 rows
+  for (int cand = fixed_march ? 1 : 0; cand <= 5; ++cand) {  // 0: tiled; 1..5: marching, 4..8 rows
     h->march = cand > 0;
     h->march_rows = cand > 0 ? 3 + cand : h->march_rows;
     if (cand > 0 && h->march_rows > fast::march_max_rows()) continue;
@@ -379,7 +398,7 @@ int autotune_precision(e2d_handle* h, int prec) {
     float ms = 0.f;
     CK(cudaEventElapsedTime(&ms, e0, e1));
     const float us = 1000.f * ms / 3.f;
-    if (us < best.us) {
+    if (us < best.us && (!fixed || h->march == fixed_march)) {
       best.us = us;
       best.march = h->march;
     }

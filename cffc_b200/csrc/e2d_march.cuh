@@ -418,6 +418,18 @@ __device__ __forceinline__ FaceGeo face_geo(double ax, double ay, double cx, dou
   return f;
 }
 
+// The same value, of which the compiler knows nothing: face<true> and
+// face<false> then contract the flux's multiplications and additions alike, so
+// a face has the same bits whichever of them its chunk takes.
+__device__ __forceinline__ float opaque(float x) {
+  asm("" : "+f"(x));
+  return x;
+}
+__device__ __forceinline__ double opaque(double x) {
+  asm("" : "+d"(x));
+  return x;
+}
+
 // Face item t of chunk k.  Items [0, ni) are the i-faces I-1/2 of rows
 // r = t / (MI+1) (I = i0+2+q, J = j0+2+r), the rest the j-faces J-1/2 of
 // slots sl in [sf_lo, h] (J = j0+2+sl, I = i0+2+q).  Both kinds share one
@@ -490,7 +502,10 @@ __device__ __forceinline__ void face(const MarchArgs& m, Smem& s, const Tile& T,
     wl = fstate(s, T, k, ls, lc, f.mx, f.my);
     wr = fstate(s, T, k, rs, rc, f.mx, f.my);
   }
-  const CState<RT> F = face_flux<ROE>(B.flux, wl, wr, RT(f.nx), RT(f.ny), g, gm1, gm1i);
+  const RT nx = opaque(RT(f.nx)), ny = opaque(RT(f.ny));
+  wl = PState<RT>{opaque(wl.d), opaque(wl.u), opaque(wl.v), opaque(wl.p)};
+  wr = PState<RT>{opaque(wr.d), opaque(wr.u), opaque(wr.v), opaque(wr.p)};
+  const CState<RT> F = face_flux<ROE>(B.flux, wl, wr, nx, ny, g, gm1, gm1i);
 #ifdef E2D_FAST
   out[0] = double(F.d) * f.l;
   out[vs] = double(F.mx) * f.l;
