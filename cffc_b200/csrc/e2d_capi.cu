@@ -233,12 +233,16 @@ bool encode3(CUtensorMap* map, void* base, uint64_t d0, uint64_t d1, uint64_t d2
 // an odd block width (their row strides must be multiples of 16 bytes), whose
 // windows the exact build copies itself.  The handle keeps the tiled stage
 // kernel when the marching kernel does not apply: a degenerate edge, an odd
-// width in the fast precisions.
+// width in the fast precisions.  A handle of odd width, which needs none of it
+// otherwise, gets its geometry (12 doubles a cell) when it first has the exact
+// precision, and stays on the tiled kernel where there is no memory for it.
 int setup_march(e2d_handle* h) {
   h->march = h->march_ok = false;
   const Blocks& B = h->B;
   h->march_plain = B.NCi % 2 != 0;
   if (!h->march_plain && !encode_fn()) return 0;
+  if (h->march_plain && h->sc.precision != E2D_PREC_FP64_EXACT) return 0;
+  h->march_tried = true;
   const int mi = fast::march_strip_cols(), wj = fast::march_window_rows();
   const int NNp = B.NNi + 1;  // NNi is odd for an even NCi
   int rc;
@@ -248,8 +252,13 @@ int setup_march(e2d_handle* h) {
       (rc = dalloc(h, &h->geomx, size_t(GEOM_NF) * h->ncell)) ||
       (rc = dalloc(h, &h->gmask, h->ncell)) ||
       (rc = dalloc(h, &h->bcside, B.nblk)) || (npad && (rc = dalloc(h, &h->nodes_pad, npad))) ||
-      (rc = dalloc(h, &degenerate, 1)))
-    return rc;
+      (rc = dalloc(h, &degenerate, 1))) {
+    if (!h->march_plain) return rc;
+    cudaGetLastError();
+    for (void* q : {(void*)h->geomx, (void*)h->gmask, (void*)h->bcside}) drop(h, q);
+    h->geomx = nullptr; h->gmask = nullptr; h->bcside = nullptr;
+    return 0;
+  }
   CK(cudaMemsetAsync(degenerate, 0, sizeof(int), h->stream));
   if (npad) CK(cudaMemsetAsync(h->nodes_pad, 0, sizeof(double) * npad, h->stream));
   // the exact build's geometry first: the fast one then writes the same mask,
@@ -348,8 +357,8 @@ bool prefers_march(int nci, int prec, int flux) {
   return nci > 18 && (flux == E2D_FLUX_ROE || nci <= 32 || nci > 36);
 }
 
-// Tunes one precision into sel_*[prec].
-int autotune_precision(e2d_handle* h, int prec) {
+// Tunes one precision into sel_*[prec], on the arrays of `a`.
+int autotune_precision(e2d_handle* h, int prec, const StageArgs& a) {
   if (!march_applies(h, prec)) return 0;  // tiled, as initialised
   const TuneKey key{h->B.nci, h->B.ncj, h->B.nblk, prec, h->sc.flux};
   {
@@ -364,18 +373,6 @@ int autotune_precision(e2d_handle* h, int prec) {
   }
   const int saved = h->sc.precision;
   h->sc.precision = prec;
-  StageArgs a{};
-  a.B = h->B;
-  a.B.dWdx = a.B.dWdy = a.B.phi = nullptr;
-  a.mode = 1;
-  a.hist = h->hist;
-  a.step = h->step;
-  a.Win = h->B.W2;
-  a.Ubase = h->B.U2;
-  a.Wout = h->B.W;
-  a.Uout = h->B.U;
-  a.res_out = h->B.dUdt;
-  a.omega = 1.0;
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
@@ -431,34 +428,65 @@ void apply_selection(e2d_handle* h) {
   h->tune_us = h->sel_us[p];
 }
 
-// Every precision is tuned when the handle is created (a handle may switch
-// between them, e2d_set_precision) on a uniform state in (W2, U2); the state
-// arrays are cleared afterwards.
-int autotune_stage(e2d_handle* h) {
-  if (!h->march_ok) return 0;
-  // "tiled" / "march": one kernel without tuning (tests and comparisons of
-  // the two kernels; "march" with its default rows per chunk, for even widths,
-  // "march_any" for odd ones too)
+// CFFC_E2D_STAGE_KERNEL when the handle is created: "tiled" / "march", one
+// kernel without tuning (tests and comparisons of the two kernels; "march" with
+// its default rows per chunk, for even widths, "march_any" for odd ones too).
+StageChoice stage_choice() {
   const char* kind = getenv("CFFC_E2D_STAGE_KERNEL");
-  if (kind && (strcmp(kind, "tiled") == 0 || strcmp(kind, "march") == 0 || strcmp(kind, "march_any") == 0)) {
-    for (int p = 0; p < 3; ++p)
-      h->sel_march[p] = march_applies(h, p) && (strcmp(kind, "march_any") == 0 ||
-                                                (strcmp(kind, "march") == 0 && !h->march_plain));
-    for (int p = 0; p < 3; ++p) h->sel_lin[p] = h->sel_march[p];
-    h->sel_rows[0] = h->sel_rows[1] = h->sel_rows[2] = fast::march_chunk_rows();
-    apply_selection(h);
-    return 0;
+  if (!kind) return STAGE_TUNED;
+  return strcmp(kind, "tiled") == 0       ? STAGE_TILED
+         : strcmp(kind, "march") == 0     ? STAGE_MARCH
+         : strcmp(kind, "march_any") == 0 ? STAGE_MARCH_ANY
+                                          : STAGE_TUNED;
+}
+void fixed_stage(e2d_handle* h) {
+  for (int p = 0; p < 3; ++p) {
+    h->sel_march[p] = march_applies(h, p) && (h->choice == STAGE_MARCH_ANY || (h->choice == STAGE_MARCH && !h->march_plain));
+    h->sel_lin[p] = h->sel_march[p];
+    h->sel_rows[p] = fast::march_chunk_rows();
   }
-  Blocks Bs = h->B;
-  Bs.W = h->B.W2;
-  Bs.U = h->B.U2;
+}
+
+// The stage that is timed: a uniform state in the Blocks' (W2, U2), stage 1 to
+// (W, U).
+int tune_args(e2d_handle* h, const Blocks& B, double* hist, int* step, StageArgs& a) {
+  a = StageArgs{};
+  a.B = B;
+  a.B.dWdx = a.B.dWdy = a.B.phi = nullptr;
+  a.mode = 1;
+  a.hist = hist;
+  a.step = step;
+  a.Win = B.W2;
+  a.Ubase = B.U2;
+  a.Wout = B.W;
+  a.Uout = B.U;
+  a.res_out = B.dUdt;
+  a.omega = 1.0;
+  Blocks Bs = B;
+  Bs.W = B.W2;
+  Bs.U = B.U2;
   const int grid = int(std::min<size_t>((h->ncell + 255) / 256, 4096));
   uniform_state_kernel<<<grid, 256, 0, h->stream>>>(Bs, (long long)h->ncell);
   CK(cudaGetLastError());
-  CK(cudaMemsetAsync(h->hist, 0, sizeof(double) * 4 * size_t(h->hist_cap) * h->B.ncase, h->stream));
+  return 0;
+}
+
+// The precisions the marching kernel is set up for (an odd width: the exact one
+// alone) are tuned when the handle is created, as a handle may switch between
+// them (e2d_set_precision); the state arrays are cleared afterwards.
+int autotune_stage(e2d_handle* h) {
+  if (!h->march_ok) return 0;
+  if (h->choice != STAGE_TUNED) {
+    fixed_stage(h);
+    apply_selection(h);
+    return 0;
+  }
   int rc;
-  if ((rc = autotune_precision(h, E2D_PREC_FP64)) || (rc = autotune_precision(h, E2D_PREC_FP32)) ||
-      (rc = autotune_precision(h, E2D_PREC_FP64_EXACT)))
+  StageArgs a;
+  CK(cudaMemsetAsync(h->hist, 0, sizeof(double) * 4 * size_t(h->hist_cap) * h->B.ncase, h->stream));
+  if ((rc = tune_args(h, h->B, h->hist, h->step, a))) return rc;
+  if ((rc = autotune_precision(h, E2D_PREC_FP64, a)) || (rc = autotune_precision(h, E2D_PREC_FP32, a)) ||
+      (rc = autotune_precision(h, E2D_PREC_FP64_EXACT, a)))
     return rc;
   for (int p = 0; p < 3; ++p)
     h->sel_lin[p] = p == E2D_PREC_FP64_EXACT ? h->sel_march[p] : march_applies(h, p);
@@ -475,6 +503,38 @@ int autotune_stage(e2d_handle* h) {
   if (h->B.phi_keep) CK(cudaMemsetAsync(h->B.phi_keep, 0, nb, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   return 0;
+}
+
+// The exact precision's set-up of a handle of odd width that is switched to
+// it: like setup_march and autotune_stage, but beside the handle's state, on
+// arrays of its own (without memory for them the tiled kernel stays).
+int setup_exact_late(e2d_handle* h) {
+  if (h->march_tried || !h->march_plain) return 0;
+  int rc = setup_march(h);
+  if (rc || !h->march_ok) return rc;
+  if (h->choice != STAGE_TUNED) {
+    fixed_stage(h);
+    return 0;
+  }
+  const size_t n = 4 * h->ncell, zeros = 8;  // status, step and a history slot
+  double* buf = nullptr;
+  if (cudaMalloc(&buf, sizeof(double) * (5 * n + h->ncell + zeros)) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  Blocks B = h->B;
+  B.W = buf; B.U = buf + n; B.W2 = buf + 2 * n; B.U2 = buf + 3 * n; B.dUdt = buf + 4 * n; B.dt = buf + 5 * n;
+  double* z = B.dt + h->ncell;
+  B.status = reinterpret_cast<int*>(z);
+  B.freeze = nullptr; B.phi_keep = nullptr;
+  B.case_of = nullptr; B.case_start = nullptr; B.case_active = nullptr; B.ncase = 1;
+  StageArgs a;
+  rc = cudaMemsetAsync(B.dt, 0, sizeof(double) * (h->ncell + zeros), h->stream) == cudaSuccess ? 0 : E2D_ERR_CUDA;
+  if (!rc) rc = tune_args(h, B, z + 2, reinterpret_cast<int*>(z + 1), a);
+  if (!rc) rc = autotune_precision(h, E2D_PREC_FP64_EXACT, a);
+  cudaFree(buf);
+  h->sel_lin[E2D_PREC_FP64_EXACT] = h->sel_march[E2D_PREC_FP64_EXACT];
+  return rc;
 }
 
 // Residual (mode 0) or Frechet product (mode 3) of the state (W, U).
@@ -900,6 +960,7 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
   if ((rc = alloc_freeze(h))) return fail(rc, h);
   if ((rc = ensure_hist(h, 64))) return fail(rc, h);
   B.dWdx = B.dWdy = B.phi = nullptr;
+  h->choice = stage_choice();
   if ((rc = setup_march(h)) || (rc = autotune_stage(h))) return fail(rc, h);
   return h;
 }
@@ -1276,6 +1337,8 @@ int e2d_set_precision(e2d_handle* h, int precision) {
   CK(cudaSetDevice(h->device));
   CK(cudaStreamSynchronize(h->stream));
   h->sc.precision = precision;
+  if (precision == E2D_PREC_FP64_EXACT)
+    if (int rc = setup_exact_late(h)) return rc;
   apply_selection(h);
   // captured launches hold the previous precision's kernels
   drop_step_graphs(h);

@@ -3,6 +3,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <vector>
 
@@ -10,6 +11,9 @@
 #include "e2d_launch.h"
 
 struct e2d_nks_state;  // NKS work arrays (e2d_nks.cu)
+
+// How a handle's stage kernel is chosen (CFFC_E2D_STAGE_KERNEL).
+enum StageChoice { STAGE_TUNED, STAGE_TILED, STAGE_MARCH, STAGE_MARCH_ANY };
 
 struct e2d_handle {
   int device = 0;
@@ -60,6 +64,8 @@ struct e2d_handle {
   double tune_us = 0.0;  // the autotuner's time of one explicit stage with the chosen kernel
   bool march_ok = false;  // geometry and tensor maps set up
   bool march_plain = false;  // odd block width: no tensor maps, exact precision only
+  bool march_tried = false;  // setup_march has run (odd widths: in the exact precision)
+  StageChoice choice = STAGE_TUNED;
   // the autotuner's choice per precision (E2D_PREC_FP64, E2D_PREC_FP32,
   // E2D_PREC_FP64_EXACT)
   bool sel_march[3] = {false, false, false};
@@ -96,6 +102,14 @@ template <class T> int dalloc(e2d_handle* h, T** p, size_t n) {
   h->allocs.push_back(q);
   *p = static_cast<T*>(q);
   return 0;
+}
+
+// Frees one of the handle's arrays (null: nothing) before the handle goes.
+inline void drop(e2d_handle* h, void* p) {
+  auto it = std::find(h->allocs.begin(), h->allocs.end(), p);
+  if (it == h->allocs.end()) return;
+  cudaFree(p);
+  h->allocs.erase(it);
 }
 
 int check_status(e2d_handle* h);
