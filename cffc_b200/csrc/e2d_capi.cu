@@ -29,10 +29,14 @@ namespace e2d_host {
   } while (0)
 
 
+// A host array's copy on the device.  On the handle's stream, like everything
+// else that makes a handle: that stream does not wait for the default one, and
+// a pageable cudaMemcpy may return before its last piece has arrived.  `src` is
+// read until the stream is synchronised (e2d_create, e2d_create_batch).
 template <class T> int upload(e2d_handle* h, T** p, const T* src, size_t n) {
   int rc = dalloc(h, p, n);
   if (rc) return rc;
-  CK(cudaMemcpy(*p, src, sizeof(T) * n, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(*p, src, sizeof(T) * n, cudaMemcpyHostToDevice, h->stream));
   return 0;
 }
 
@@ -640,11 +644,11 @@ int alloc_freeze(e2d_handle* h) {
   if ((rc = dalloc(h, &h->freeze, size_t(h->B.ncase))) || (rc = dalloc(h, &h->first, 1))) return rc;
   if (!h->B.phi_keep) {
     if ((rc = dalloc(h, &h->B.phi_keep, 4 * h->ncell))) return rc;
-    CK(cudaMemset(h->B.phi_keep, 0, sizeof(double) * 4 * h->ncell));
+    CK(cudaMemsetAsync(h->B.phi_keep, 0, sizeof(double) * 4 * h->ncell, h->stream));
   }
-  const int one = 1;
-  CK(cudaMemset(h->freeze, 0, sizeof(int) * h->B.ncase));
-  CK(cudaMemcpy(h->first, &one, sizeof(int), cudaMemcpyHostToDevice));
+  static const int one = 1;
+  CK(cudaMemsetAsync(h->freeze, 0, sizeof(int) * h->B.ncase, h->stream));
+  CK(cudaMemcpyAsync(h->first, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
   h->B.freeze = h->freeze;
   return 0;
 }
@@ -920,11 +924,10 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
       (rc = dalloc(h, &B.dt, h->ncell)) || (rc = dalloc(h, &B.status, 2)) ||
       (rc = dalloc(h, &h->step, 2)) || (rc = dalloc(h, &h->part, size_t(3) * B.nblk)))
     return fail(rc, h);
-  if (cudaMemset(B.W, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(B.U, 0, sizeof(double) * 4 * h->ncell) ||
-      cudaMemset(B.W2, 0, sizeof(double) * 4 * h->ncell) ||
-      cudaMemset(B.U2, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(B.dUdt, 0, sizeof(double) * 4 * h->ncell) ||
-      cudaMemset(B.dt, 0, sizeof(double) * h->ncell) || cudaMemset(B.status, 0, sizeof(int) * 2) ||
-      cudaMemset(h->step, 0, 2 * sizeof(int)))
+  auto clear = [&](void* q, size_t bytes) { return cudaMemsetAsync(q, 0, bytes, h->stream) != cudaSuccess; };
+  const size_t state = sizeof(double) * 4 * h->ncell;
+  if (clear(B.W, state) || clear(B.U, state) || clear(B.W2, state) || clear(B.U2, state) || clear(B.dUdt, state) ||
+      clear(B.dt, sizeof(double) * h->ncell) || clear(B.status, sizeof(int) * 2) || clear(h->step, 2 * sizeof(int)))
     return fail(E2D_ERR_CUDA, h);
   unsigned char* flags = nullptr;
   double2* nrm = nullptr;
@@ -934,13 +937,11 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
   B.edge_nrm = nrm;
   if (sc->n_stage >= 3) {
     if ((rc = dalloc(h, &h->W3, 4 * h->ncell)) || (rc = dalloc(h, &h->U3, 4 * h->ncell))) return fail(rc, h);
-    if (cudaMemset(h->W3, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(h->U3, 0, sizeof(double) * 4 * h->ncell))
-      return fail(E2D_ERR_CUDA, h);
+    if (clear(h->W3, state) || clear(h->U3, state)) return fail(E2D_ERR_CUDA, h);
   }
   if (stage_plan(*sc, sc->n_stage).rk4) {
     if ((rc = dalloc(h, &h->R1, 4 * h->ncell)) || (rc = dalloc(h, &h->R2, 4 * h->ncell))) return fail(rc, h);
-    if (cudaMemset(h->R1, 0, sizeof(double) * 4 * h->ncell) || cudaMemset(h->R2, 0, sizeof(double) * 4 * h->ncell))
-      return fail(E2D_ERR_CUDA, h);
+    if (clear(h->R1, state) || clear(h->R2, state)) return fail(E2D_ERR_CUDA, h);
   }
   if (sc->rs_epsilon > 0.0) {
     // the smoothing region and its zero ring, [4][ncj][nci] doubles per block,
@@ -962,6 +963,7 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
   B.dWdx = B.dWdy = B.phi = nullptr;
   h->choice = stage_choice();
   if ((rc = setup_march(h)) || (rc = autotune_stage(h))) return fail(rc, h);
+  if (cudaStreamSynchronize(h->stream) != cudaSuccess) return fail(E2D_ERR_CUDA, h);
   return h;
 }
 
@@ -1028,7 +1030,8 @@ e2d_handle* e2d_create_batch(const e2d_blocks_desc* cases, int ncase, const e2d_
   // the step history holds one slot per case and step
   const int cap = h->hist_cap;
   h->hist_cap = 0;
-  if ((rc = ensure_hist(h, cap)) || (rc = alloc_freeze(h))) {
+  if ((rc = ensure_hist(h, cap)) || (rc = alloc_freeze(h)) ||
+      (rc = cudaStreamSynchronize(h->stream) == cudaSuccess ? 0 : E2D_ERR_CUDA)) {
     if (err) *err = rc;
     e2d_destroy(h);
     return nullptr;

@@ -1059,7 +1059,7 @@ int ilu_setup(e2d_handle* h, int level) {
     void* q = nullptr;
     if (cudaMalloc(&q, bytes ? bytes : 1) != cudaSuccess) return E2D_ERR_NOMEM;
     s->ilu_allocs.push_back(q);
-    if (src && bytes && cudaMemcpy(q, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return E2D_ERR_CUDA;
+    if (src && bytes && cudaMemcpyAsync(q, src, bytes, cudaMemcpyHostToDevice, h->stream) != cudaSuccess) return E2D_ERR_CUDA;
     *dst = q;
     return 0;
   };
@@ -1547,7 +1547,7 @@ static bool params_ok(const e2d_nks_params& p) {
 extern "C" int e2d_nks(e2d_handle* h, const e2d_nks_params* p, e2d_nks_step* hist, int* n_steps) {
   if (!h) return nks_run(h, p, hist, n_steps);
   if (!h->subs.empty()) return p ? composite_nks(h, p, hist, n_steps) : E2D_ERR_ARG;
-  if (h->freeze && cudaMemset(h->freeze, 0, sizeof(int) * h->B.ncase) != cudaSuccess) return E2D_ERR_CUDA;
+  if (h->freeze && cudaMemsetAsync(h->freeze, 0, sizeof(int) * h->B.ncase, h->stream) != cudaSuccess) return E2D_ERR_CUDA;
   const int* saved = h->B.freeze;
   h->B.freeze = nullptr;
   const int rc = nks_run(h, p, hist, n_steps);
