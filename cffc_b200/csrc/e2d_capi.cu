@@ -950,8 +950,7 @@ e2d_handle* e2d_create(const e2d_blocks_desc* d, const e2d_scheme* sc, int devic
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
     if (bytes <= size_t(max_smem) &&
-        cudaFuncSetAttribute(residual_smoothing_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(bytes)) == cudaSuccess) {
+        allow_smem(residual_smoothing_kernel<true>) == cudaSuccess) {
       h->smooth_smem = bytes;
     } else {
       cudaGetLastError();

@@ -104,6 +104,19 @@ template <class T> int dalloc(e2d_handle* h, T** p, size_t n) {
   return 0;
 }
 
+// Lets the kernel be launched with all the shared memory that the device has
+// beside the kernel's static part.  The limit belongs to the process: one set to
+// a handle's own need would refuse the launches of another with larger blocks.
+template <class K> cudaError_t allow_smem(K* kernel) {
+  int dev = 0, optin = 0;
+  cudaFuncAttributes fa{};
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) || (e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) ||
+      (e = cudaFuncGetAttributes(&fa, kernel)))
+    return e;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - int(fa.sharedSizeBytes));
+}
+
 // Frees one of the handle's arrays (null: nothing) before the handle goes.
 inline void drop(e2d_handle* h, void* p) {
   auto it = std::find(h->allocs.begin(), h->allocs.end(), p);

@@ -1118,7 +1118,7 @@ int ilu_setup(e2d_handle* h, int level) {
     void* w = nullptr;
     if (s->ilu_solve_smem + sa.sharedSizeBytes <= size_t(optin) && up(nullptr, svals, &w) == 0) {
       E2D_CK(cudaMemsetAsync(w, 0, svals, h->stream));
-      E2D_CK(cudaFuncSetAttribute(solver, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s->ilu_solve_smem)));
+      E2D_CK(allow_smem(solver));
       D.svals = static_cast<double*>(w);
       streamed = P.xstages <= ILU_MAX_STAGES && s->ilu_levels_smem + xa.sharedSizeBytes <= size_t(optin);
     }
@@ -1129,7 +1129,7 @@ int ilu_setup(e2d_handle* h, int level) {
     if ((rc = up(nullptr, sizeof(double) * 16 * size_t(P.nrow) * P.maxrow * nblk, &v))) return rc;
     D.vals = static_cast<double*>(v);
     D.nvals = P.nrow * P.maxrow;
-    E2D_CK(cudaFuncSetAttribute(ilu_levels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(s->ilu_levels_smem)));
+    E2D_CK(allow_smem(ilu_levels_kernel));
     s->ilu_level = level;
     return 0;
   }
@@ -1143,7 +1143,7 @@ int ilu_setup(e2d_handle* h, int level) {
   const size_t smem = sizeof(double) * 4 * size_t(P.nrow) + sizeof(int4) * 2 * size_t(P.nrow) +
                       sizeof(int) * size_t(P.nflev + P.nblev + 2);
   if (smem <= size_t(optin)) {
-    E2D_CK(cudaFuncSetAttribute(ilu_apply_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    E2D_CK(allow_smem(ilu_apply_kernel<true>));
     s->ilu_smem = smem;
   } else {
     if ((rc = up(nullptr, sizeof(double) * 4 * size_t(P.nrow) * nblk, &w))) return rc;
@@ -1155,8 +1155,7 @@ int ilu_setup(e2d_handle* h, int level) {
   cudaFuncAttributes fa{};
   E2D_CK(cudaFuncGetAttributes(&fa, ilu_factor_kernel));  // its static shared memory counts too
   if (s->ilu_factor_smem + fa.sharedSizeBytes > size_t(optin)) return E2D_ERR_ARG;
-  E2D_CK(cudaFuncSetAttribute(ilu_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(s->ilu_factor_smem)));
+  E2D_CK(allow_smem(ilu_factor_kernel));
   s->ilu_level = level;
   return 0;
 }
