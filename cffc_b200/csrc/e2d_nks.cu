@@ -1103,7 +1103,8 @@ int ilu_setup(e2d_handle* h, int level) {
   // most 8 entries a side), the levels at most 32 rows, the buffers fit and
   // there is memory for their copy of the factors (padding zero); and with
   // them the streamed factorization where its buffers fit too (not for level 4
-  // on blocks of 64 x 32).  Else the kernels that work on the factors in HBM.
+  // on blocks of 64 x 32).  Else, and where there is no memory for what the
+  // streamed kernels keep beside, the kernels that work on the factors in HBM.
   // Measured on B200, 12 blocks of 32 x 32, ILU(2): factorization 885 -> 378 us,
   // solve 173 -> 62 us.
   const IluSolve solver = P.nsvals ? ilu_solver(P.sent) : nullptr;
@@ -1124,20 +1125,29 @@ int ilu_setup(e2d_handle* h, int level) {
     }
     cudaGetLastError();
   }
-  if (streamed) {
-    void* v = nullptr;
-    if ((rc = up(nullptr, sizeof(double) * 16 * size_t(P.nrow) * P.maxrow * nblk, &v))) return rc;
+  void* v = nullptr;
+  if (streamed && up(nullptr, sizeof(double) * 16 * size_t(P.nrow) * P.maxrow * nblk, &v) == 0) {
     D.vals = static_cast<double*>(v);
     D.nvals = P.nrow * P.maxrow;
     E2D_CK(allow_smem(ilu_levels_kernel));
     s->ilu_level = level;
     return 0;
   }
-  void *v0, *v1, *w;
-  if ((rc = up(nullptr, sizeof(double) * 16 * size_t(P.nnz) * nblk, &v0)) ||
-      (rc = up(nullptr, sizeof(double) * 16 * size_t(P.nrow) * nblk, &v1)))
-    return rc;
-  D.vals = static_cast<double*>(v0); D.dinv = static_cast<double*>(v1);
+  // the factors, then the inverted diagonals
+  void *v0 = nullptr, *w;
+  const size_t nfac = 16 * size_t(P.nnz) * nblk, ninv = 16 * size_t(P.nrow) * nblk;
+  rc = up(nullptr, sizeof(double) * (nfac + ninv), &v0);
+  if (rc && D.svals) {
+    cudaGetLastError();
+    E2D_CK(cudaStreamSynchronize(h->stream));
+    s->ilu_allocs.erase(std::find(s->ilu_allocs.begin(), s->ilu_allocs.end(), (void*)D.svals));
+    cudaFree(D.svals);
+    D.svals = nullptr;
+    rc = up(nullptr, sizeof(double) * (nfac + ninv), &v0);
+  }
+  if (rc) return rc;
+  cudaGetLastError();
+  D.vals = static_cast<double*>(v0); D.dinv = D.vals + nfac;
   D.nvals = P.nnz;
   // a block's vector in shared memory when it fits, else a global work array
   const size_t smem = sizeof(double) * 4 * size_t(P.nrow) + sizeof(int4) * 2 * size_t(P.nrow) +
