@@ -851,7 +851,7 @@ __global__ void __launch_bounds__(ILU_APPLY_THREADS) ilu_apply_kernel(Blocks B, 
 // (k + 1) ncj of them each way.  With a warp or two a level every instruction
 // counts, so a thread loads the next level's blocks and cells into registers
 // before the additions of this one, the tables are 16-bit cells read 16 bytes
-// at once, and every thread works (those past the last row repeat it, unwritten): 12 blocks
+// at once, and every thread works (those past the last row repeat it): 12 blocks
 // of 32 x 32, ILU(2), 173 -> 62 us; the same ring with the blocks read when their
 // level begins took 170.
 constexpr int ILU_STAGES = 4;
@@ -939,7 +939,6 @@ __global__ void __launch_bounds__(32 * (1 + ILU_SOLVE_ROWS / 8)) ilu_solve_kerne
     }
   } else {
     const int k = tid & 3, q0 = tid & 28, r = min(tid >> 2, R - 1);
-    const bool mine = (tid >> 2) < R;  // of the threads on one row the first four write it: none reads another's result
     // level t from `c` while level t + 1 is loaded into `n`
     auto level = [&](const SolveRow<M>& c, SolveRow<M>& n, int t) {
       double2 ya[M], yb[M];
@@ -972,7 +971,8 @@ __global__ void __launch_bounds__(32 * (1 + ILU_SOLVE_ROWS / 8)) ilu_solve_kerne
         acc = acc + y2 * c.a[M][1].x;
         acc = acc + y3 * c.a[M][1].y;
       }
-      if (mine) *own = acc;
+      __syncwarp();  // the threads on the last row have all read its values (their stores alone by its four: 1 % slower)
+      *own = acc;
       __syncwarp();
       if (t + 1 < nlev && (tid & 31) == 0) tc::mbar_arrive(&empty[q]);
       ok = solve_barrier(nsolve, ok);
