@@ -74,13 +74,4 @@ __device__ __forceinline__ PState<double> wo_at(const double* wo, int b, int len
   return w;
 }
 
-__device__ __forceinline__ void ghost_set(const Blocks& B, int b, int i, int j, const PState<double>& w) {
-  stW(B, b, i, j, w);
-  stU(B, b, i, j, U_of_W(w, B.gm1i));
-}
-__device__ __forceinline__ void ghost_copy(const Blocks& B, int b, int id, int jd, int is, int js) {
-  stW(B, b, id, jd, ldW(B, b, is, js));
-  stU(B, b, id, jd, ldU(B, b, is, js));
-}
-
 }  // namespace e2d

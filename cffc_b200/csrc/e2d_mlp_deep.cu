@@ -796,7 +796,6 @@ e2d_mlp_deep* e2d_mlp_deep_create(uint64_t seed, int* err) {
   e2d_mlp_deep* d = new e2d_mlp_deep;
   cudaGetDevice(&d->device);
   cudaDeviceGetAttribute(&d->sms, cudaDevAttrMultiProcessorCount, d->device);
-  std::vector<void*> fixed;
   bool ok = cudaMalloc(&d->p, 4 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->g, 4 * size_t(NPARAM)) == cudaSuccess &&
             cudaMalloc(&d->m, 4 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->v, 4 * size_t(NPARAM)) == cudaSuccess &&
             cudaMalloc(&d->wk, 2 * size_t(NPARAM)) == cudaSuccess && cudaMalloc(&d->wt, 2 * size_t(NPARAM)) == cudaSuccess &&
