@@ -137,7 +137,10 @@ e2d_handle *e2d_create(const e2d_blocks_desc *desc, const e2d_scheme *scheme,
  * Their blocks are laid end to end in case order; every entry point then
  * works on all cases at once, with per-case time-step minima, residual
  * norms, histories and Newton-Krylov solves, and gives each case the same
- * result bit for bit as a handle of that case alone.  Cases of different
+ * result bit for bit as a handle of that case alone (of explicit runs the
+ * residual norms to 1e-12: they are summed atomically; and in FP64 and FP32 a
+ * batch of which one case has an edge of length zero runs all of them on the
+ * tiled kernel, which rounds differently).  Cases of different
  * block dimensions run as one batch per block shape behind this handle; the
  * host arrays (states, residuals, local time steps) are then each case's
  * array in its own shape, concatenated in case order, and
@@ -352,14 +355,19 @@ int e2d_fastmath_check(const double *x, int n, double *out);
  * tolerance on the same state.  No reference counterpart. */
 int e2d_set_precision(e2d_handle *h, int precision);
 
-/* The stage kernel the handle's autotuner chose when the handle was created:
+/* The kernel of the handle's explicit stages in its current precision:
  * *kernel 0 = the tiled kernel, 1 = the column-marching kernel with *rows
- * rows per chunk; *us the tuner's time of one explicit stage with it (0 when
- * no tuning ran: a degenerate edge, or an odd block width outside exact
- * precision, where the tiled kernel is the only one).  Any pointer may be NULL.  The environment variable
- * CFFC_E2D_STAGE_KERNEL=tiled or =march, read when a handle is created,
- * fixes the kernel without tuning (the marching kernel still only where it
- * applies).  No reference counterpart. */
+ * rows per chunk; *us the autotuner's time of one explicit stage with it (0
+ * when no tuning ran: a degenerate edge, or an odd block width outside exact
+ * precision, where the tiled kernel is the only one).  In FP64 and FP32, where
+ * the two round differently, the kernel follows from the block width, the
+ * precision and the flux, and the autotuner chooses the rows alone; in exact
+ * precision it chooses both.  It runs when a handle is created or, for an odd
+ * width, first has the exact precision.  Any pointer may be NULL.  The
+ * environment variable CFFC_E2D_STAGE_KERNEL, read when a handle is created,
+ * fixes the kernel without tuning: =tiled, =march (the marching kernel on even
+ * widths without a degenerate edge) or =march_any (also on odd widths in exact
+ * precision).  No reference counterpart. */
 int e2d_stage_config(e2d_handle *h, int *kernel, int *rows, double *us);
 
 /* The deep warm-start network (library extension, no reference
