@@ -169,6 +169,7 @@ cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
       m.geom = ex ? h->geomx : h->geom;
       m.mask = h->gmask;
       m.bcside = h->bcside;
+      m.edges = h->march_edges;
       // update inputs by TMA: explicit stages over U or U2 whose second
       // stage adds to dUdt (RK4's slot combination reads global memory)
       const bool ubase = a.Ubase == h->B.U || a.Ubase == h->B.U2;
@@ -250,30 +251,31 @@ int setup_march(e2d_handle* h) {
   const int mi = fast::march_strip_cols(), wj = fast::march_window_rows();
   const int NNp = B.NNi + 1;  // NNi is odd for an even NCi
   int rc;
-  int* degenerate = nullptr;
+  int* flags = nullptr;  // a degenerate edge, a block side that sets face states
   const size_t npad = h->march_plain ? 0 : size_t(B.nblk) * 2 * B.NNj * NNp;
   if ((!h->march_plain && (rc = dalloc(h, &h->geom, size_t(GEOM_NF) * h->ncell))) ||
       (rc = dalloc(h, &h->geomx, size_t(GEOM_NF) * h->ncell)) ||
       (rc = dalloc(h, &h->gmask, h->ncell)) ||
       (rc = dalloc(h, &h->bcside, B.nblk)) || (npad && (rc = dalloc(h, &h->nodes_pad, npad))) ||
-      (rc = dalloc(h, &degenerate, 1))) {
+      (rc = dalloc(h, &flags, 2))) {
     if (!h->march_plain) return rc;
     cudaGetLastError();
     for (void* q : {(void*)h->geomx, (void*)h->gmask, (void*)h->bcside}) drop(h, q);
     h->geomx = nullptr; h->gmask = nullptr; h->bcside = nullptr;
     return 0;
   }
-  CK(cudaMemsetAsync(degenerate, 0, sizeof(int), h->stream));
+  CK(cudaMemsetAsync(flags, 0, 2 * sizeof(int), h->stream));
   if (npad) CK(cudaMemsetAsync(h->nodes_pad, 0, sizeof(double) * npad, h->stream));
   // the exact build's geometry first: the fast one then writes the same mask,
-  // side bits and padded nodes again, and both flag degenerate edges
-  CK(exact::launch_geometry(B, h->geomx, h->gmask, h->bcside, degenerate, NNp, h->nodes_pad, h->stream));
+  // side bits and padded nodes again, and both set the flags
+  CK(exact::launch_geometry(B, h->geomx, h->gmask, h->bcside, flags, NNp, h->nodes_pad, h->stream));
   if (!h->march_plain)
-    CK(fast::launch_geometry(B, h->geom, h->gmask, h->bcside, degenerate, NNp, h->nodes_pad, h->stream));
-  int deg = 0;
-  CK(cudaMemcpyAsync(&deg, degenerate, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CK(fast::launch_geometry(B, h->geom, h->gmask, h->bcside, flags, NNp, h->nodes_pad, h->stream));
+  int found[2] = {0, 0};
+  CK(cudaMemcpyAsync(found, flags, sizeof(found), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
-  if (deg) return 0;
+  h->march_edges = found[1] != 0;
+  if (found[0]) return 0;
   if (!h->march_plain) {
     const uint32_t wi = mi + 4, nwi = mi + 6;
     bool ok = encode3(&h->tmW[0], B.W, B.NCi, B.NCj, 4ull * B.nblk, wi, wj, 4) &&

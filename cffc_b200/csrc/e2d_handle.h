@@ -47,6 +47,7 @@ struct e2d_handle {
   CUtensorMap tmGx, tmGAx, tmGFx;  // the exact build's geometry: window, update inputs
   unsigned char* gmask = nullptr;
   unsigned char* bcside = nullptr;  // per block: sides with face-setting BCs (marching kernel)
+  bool march_edges = false;         // a block has one
   // A batch whose cases have different block shapes holds no blocks of its
   // own: one uniform sub-batch per shape, every call dispatched to them.
   // Per case (in the order given): its sub-batch and index there, and the

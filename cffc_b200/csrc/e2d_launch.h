@@ -14,7 +14,7 @@ int tile_j();
 // column-marching stage kernel in the reference's arithmetic and its geometry
 cudaError_t launch_march(const MarchArgs& m, int grid, cudaStream_t st);
 int march_ctas_per_sm();
-cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, unsigned char* bcside, int* degenerate,
+cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, unsigned char* bcside, int* flags,
                             int NNp, double* nodes_pad, cudaStream_t st);
 }  // namespace exact
 namespace fast {
@@ -30,7 +30,7 @@ int march_chunk_rows();
 int march_max_rows();
 int march_window_rows();
 int march_chunks(int ncj, int ch);
-cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, unsigned char* bcside, int* degenerate,
+cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, unsigned char* bcside, int* flags,
                             int NNp, double* nodes_pad, cudaStream_t st);
 }  // namespace fast
 namespace f32 {

@@ -46,3 +46,17 @@ def test_same_bits_for_any_number_of_blocks(nci, ncj, flux, precision, monkeypat
     monkeypatch.setenv("CFFC_E2D_STAGE_KERNEL", "march" if kernel else "tiled")  # the default rows per chunk
     _, _, (W1, U1) = march(capi.Handle(bs), 5)
     assert np.array_equal(W1, W) and np.array_equal(U1, U)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("flux", [cases.FLUX_ROE, cases.FLUX_HLLC])
+def test_periodic_and_walled_cases_in_one_batch(flux, precision):
+    """A handle with walls takes another instance of the FP32 Roe kernel than a
+    periodic one alone."""
+    sc = cases.Scheme(cfl=0.4, precision=precision, flux=flux)
+    fam = [cases.periodic_box_bumps(nb=3, nc=32, seed=4, scheme=sc), block_set(2, 3, 32, 32, precision, flux)]
+    _, hist, states = march(capi.BatchHandle(fam), 8)
+    for c, bs in enumerate(fam):
+        _, h1, (_, U) = march(capi.Handle(bs), 8)
+        assert np.array_equal(bs.interior(states[c][1]), bs.interior(U)), c
+        assert np.array_equal(hist[:, c, 0], h1[:, 0])
