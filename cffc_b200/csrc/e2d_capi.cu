@@ -169,7 +169,6 @@ cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
       m.geom = ex ? h->geomx : h->geom;
       m.mask = h->gmask;
       m.bcside = h->bcside;
-      m.edges = h->march_edges;
       // update inputs by TMA: explicit stages over U or U2 whose second
       // stage adds to dUdt (RK4's slot combination reads global memory)
       const bool ubase = a.Ubase == h->B.U || a.Ubase == h->B.U2;
@@ -187,9 +186,9 @@ cudaError_t launch_stage_args(e2d_handle* h, StageArgs& a) {
       m.cps = fast::march_chunks(h->B.ncj, m.ch);
       m.nchunk = (long long)m.strips * m.cps * h->B.nblk;
       const int grid = int(std::min<long long>(m.nchunk, h->march_grid));
-      if (ex) return exact::launch_march(m, grid, h->stream);
-      return h->sc.precision == E2D_PREC_FP32 ? f32::launch_march(m, grid, h->stream)
-                                              : fast::launch_march(m, grid, h->stream);
+      if (ex) return exact::launch_march(m, grid, h->march_edges, h->stream);
+      return h->sc.precision == E2D_PREC_FP32 ? f32::launch_march(m, grid, h->march_edges, h->stream)
+                                              : fast::launch_march(m, grid, h->march_edges, h->stream);
     }
   }
   int ti, tj;

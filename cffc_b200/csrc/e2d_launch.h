@@ -12,7 +12,7 @@ size_t stage_smem_bytes();
 int tile_i();
 int tile_j();
 // column-marching stage kernel in the reference's arithmetic and its geometry
-cudaError_t launch_march(const MarchArgs& m, int grid, cudaStream_t st);
+cudaError_t launch_march(const MarchArgs& m, int grid, bool edges, cudaStream_t st);
 int march_ctas_per_sm();
 cudaError_t launch_geometry(const Blocks& B, double* geom, unsigned char* mask, unsigned char* bcside, int* flags,
                             int NNp, double* nodes_pad, cudaStream_t st);
@@ -23,7 +23,7 @@ size_t stage_smem_bytes();
 int tile_i();
 int tile_j();
 // column-marching stage kernel (e2d_march.cuh) and its per-handle geometry
-cudaError_t launch_march(const MarchArgs& m, int grid, cudaStream_t st);
+cudaError_t launch_march(const MarchArgs& m, int grid, bool edges, cudaStream_t st);
 int march_ctas_per_sm();
 int march_strip_cols();
 int march_chunk_rows();
@@ -38,7 +38,7 @@ cudaError_t launch_stage(const StageArgs& a, cudaStream_t st);
 size_t stage_smem_bytes();
 int tile_i();
 int tile_j();
-cudaError_t launch_march(const MarchArgs& m, int grid, cudaStream_t st);
+cudaError_t launch_march(const MarchArgs& m, int grid, bool edges, cudaStream_t st);
 int march_ctas_per_sm();
 }  // namespace f32
 

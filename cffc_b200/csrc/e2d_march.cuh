@@ -1001,10 +1001,11 @@ cudaError_t launch_march_flux(const MarchArgs& m, int grid, cudaStream_t st) {
     default: return cudaErrorInvalidValue;
   }
 }
-cudaError_t launch_march(const MarchArgs& m, int grid, cudaStream_t st) {
+// edges: a block has a side whose boundary condition sets the face state
+cudaError_t launch_march(const MarchArgs& m, int grid, bool edges, cudaStream_t st) {
   if (m.a.B.flux != E2D_FLUX_ROE) return launch_march_flux<false, false>(m, grid, st);
 #ifdef E2D_FP32
-  if (m.edges) return launch_march_flux<true, true>(m, grid, st);
+  if (edges) return launch_march_flux<true, true>(m, grid, st);
 #endif
   return launch_march_flux<true, false>(m, grid, st);
 }

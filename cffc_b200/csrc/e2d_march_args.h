@@ -50,7 +50,6 @@ struct MarchArgs {
   const double* geom;
   const unsigned char* mask;
   const unsigned char* bcside;  // per block: sides with face-setting boundary conditions (bits W E S N)
-  int edges;                    // 1: a block has such a side
   int strips;        // column strips per block
   int ch;            // rows of a chunk (the last chunk of a strip may hold up to 8)
   int cps;           // chunks per strip
