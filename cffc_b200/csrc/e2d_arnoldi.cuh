@@ -22,9 +22,9 @@
 // 2.6 us).
 //
 // Bound: the latency of a reduction, j + 2 of them a step one after another:
-// about 1.4 us each in a cluster (2,750 cycles: 880 the update and product, 500
-// the warps' sums, 600 the exchange, 370 the final sum and barriers), 4 us
-// across the GPU, against 4-5 us for a launch of axpy_dot_kernel.  Measured on
+// about 1.3 us each in a cluster (of 2,350 cycles counted 880 for the update and
+// product, 500 the warps' sums, 600 the exchange, 370 the final sum and barriers),
+// 3.9 us across the GPU, against 4-5 us for a launch of axpy_dot_kernel.  Measured on
 // B200: 5 Newton steps on 12,288 cells, block Jacobi 50.5 -> 28.6 ms; 6 on 98,304
 // cells 29.8 -> 21.6 ms.  A counter and fences instead of tagged sums took 5.9
 // us a round across the GPU, acquiring polls 6.8.

@@ -534,7 +534,7 @@ constexpr uint32_t ILU_WAIT = 1u << 22;
 //
 // Bound: a level's chain (per L entry the multiplier and its updates, then the
 // 4 x 4 inverse of one thread).  Measured on B200, ILU(2) on blocks of 32 x 32 (125
-// levels): 12 blocks 885 -> 378 us, 182 blocks 1,756 -> 462 us.
+// levels): 12 blocks 781 -> 375 us, 182 blocks 1,737 -> 457 us.
 __global__ void __launch_bounds__(32 * (1 + ILU_SOLVE_ROWS / 2)) ilu_levels_kernel(Blocks B, IluDev D) {
   extern __shared__ __align__(16) unsigned char buf[];
   __shared__ uint64_t full[ILU_MAX_STAGES], done[ILU_MAX_STAGES];
@@ -852,8 +852,8 @@ __global__ void __launch_bounds__(ILU_APPLY_THREADS) ilu_apply_kernel(Blocks B, 
 // counts, so a thread loads the next level's blocks and cells into registers
 // before the additions of this one, the tables are 16-bit cells read 16 bytes
 // at once, and every thread works (those past the last row repeat it): 12 blocks
-// of 32 x 32, ILU(2), 173 -> 62 us; the same ring with the blocks read when their
-// level begins took 170.
+// of 32 x 32, ILU(2), 171 -> 90 us, 182 blocks 272 -> 101; the same ring with the
+// blocks read when their level begins was no faster than the kernel before.
 constexpr int ILU_STAGES = 4;
 
 // Shared memory: the block's vector with a zero and a padding cell, the ring.

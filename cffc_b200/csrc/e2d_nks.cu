@@ -1105,8 +1105,8 @@ int ilu_setup(e2d_handle* h, int level) {
   // them the streamed factorization where its buffers fit too (not for level 4
   // on blocks of 64 x 32).  Else, and where there is no memory for what the
   // streamed kernels keep beside, the kernels that work on the factors in HBM.
-  // Measured on B200, 12 blocks of 32 x 32, ILU(2): factorization 885 -> 378 us,
-  // solve 173 -> 62 us.
+  // Measured on B200, 12 blocks of 32 x 32, ILU(2): factorization 781 -> 375 us,
+  // solve 171 -> 90 us.
   const IluSolve solver = P.nsvals ? ilu_solver(P.sent) : nullptr;
   bool streamed = false;  // the factorization
   if (solver) {
